@@ -148,6 +148,12 @@ struct AxisJob {
   double* part;              // nlines * ntile * nchunk * 64 partial sums (nchunk > 1)
   unsigned int* cnt;         // nlines * ntile arrival counters (nchunk > 1)
   // two-level passes (REDFT00 / RODFT00 kinds with D = A * B)
+  // tensor-core passes: maxima over the lines that an x pass leaves for the y
+  // pass that reads its output (high words of |.|), or null
+  unsigned* cmax;
+  const unsigned* lmax;
+  const struct TcMat* tc;    // its matrix when the job runs on the tensor cores
+  int tc_decided;            // 1: a y pass that goes as its x pass does
   int A, B;                  // 0 when the direct sum is used
   double* cs;                // nlines * B * (A + 1) * 2 partial cos/sin sums
 };
@@ -315,6 +321,24 @@ struct AxisJob;
 // FP64 instructions per line of the FFT pass of job J with plan f.
 double fft_line_cost(const FftPlanInfo& f);
 
+// Digits of a transform matrix for the tensor-core passes (tcx.cu): BF16,
+// [parity][digit][row][kp].  Form 0 (F): every output k <= D / 2 of the even
+// and odd inputs; form 1 (T): even and odd outputs k < nout of the folded
+// inputs j <= D / 2.
+struct TcMat {
+  int D = 0, form = 0, sin_kind = 0;
+  double scale = 0.0;        // interior input weight times interior output scale
+  int nout = 0;              // outputs it can give
+  int nrows = 0, kp = 0;     // rows per parity, terms per parity (padded)
+  int ew = 0;                // entries are scaled by 2^-ew
+  const void* dev = nullptr;
+};
+constexpr int kTcMaxD = 6200;  // the fixed-point sums of tcx.cu hold two parities of this many terms
+constexpr int kTcMats = 16;
+// room for the maxima of kMaxJobs x passes and an error flag at the start of
+// the scratch; the two-level passes keep off it
+constexpr long long kTcMaxBytes = ((long long)kMaxJobs * (kTcMaxD + 8) * 4 + 64 + 1023) / 1024 * 1024;
+
 struct Tables {
   int n1, n2, nd1, nd2, n3_add;
   int nsm;                   // SMs of the device (sizes the split of the sums)
@@ -338,6 +362,10 @@ struct Tables {
   // FFT plans of the axis lengths (x and y, free-surface and dealiased grids)
   FftPlanInfo fft[4];
   int nfft = 0;
+  // matrices of the tensor-core passes (3-D tanks); their digits and partial
+  // sums use the scratch cs
+  TcMat tc[kTcMats];
+  int ntc = 0;
 };
 
 // The plan of tb for J's length when the FFT pass should run J (a REDFT00 /
@@ -348,6 +376,19 @@ struct Tables {
 const FftPlanInfo* fft_choice(const AxisJob& J, const Tables& tb, double cost_other);
 // Launch the FFT passes of b's jobs, job i with plan[i].
 void launch_fft_jobs(const AxisBatch& b, const FftPlanInfo* const* plan, const Tables& tb, cudaStream_t st);
+// Tensor-core passes (tcx.cu).  build_tc_matrix makes a matrix on the device
+// (appended to `allocs`).  tc_choose sets AxisJob::tc of the requests that
+// should run there, given the time (us) of their passes elsewhere: jobs[p][i]
+// and alt[p][i] are pass p of request i, p = 0 the x and 1 the y pass, or a y
+// pass alone (npass = 1).  launch_tc_jobs runs the jobs of a batch (all x or
+// all y passes, every one with its matrix), false if one of them does not fit
+// the scratch.
+bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<void*>& allocs, TcMat* out);
+// Scratch (doubles) that holds the digits of `first` lines of `second` points
+// for each of the given pairs, one at a time.
+long long tc_scratch_doubles(int nsm, const std::vector<std::pair<long long, int>>& lines);
+void tc_choose(AxisJob* const* jobs, const double* const* alt, int npass, int n, const Tables& tb);
+bool launch_tc_jobs(const AxisBatch& b, const Tables& tb, cudaStream_t st);
 // Layout tuning of the FFT passes: with recording on (this thread), launches
 // whose batch has no tuned layout are recorded; fft_tune_run times the
 // layouts of the recorded batches on `st` (outside any capture) and keeps

@@ -836,6 +836,11 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
     // two-level pass scratch: up to kMaxJobs x-pass jobs over nd2 lines,
     // B (A+1) 2 <= 2 (D+2) doubles per line for any factor pair
     c.tb.cs_cap = (long long)kMaxJobs * std::max(nd2, n2) * 4LL * (std::max(nd1, n1) + 2);
+    // the tensor-core passes of a 3-D tank keep their digits and sums there:
+    // kMaxJobs fields of the dealiased grid, or the y lines of phiadd_SL
+    if (n2 > 1)
+      c.tb.cs_cap = std::max(c.tb.cs_cap, tc_scratch_doubles(c.tb.nsm, {{kMaxJobs * nd2, nd1}, {kMaxJobs * nd1, nd2},
+                                                                        {n1 * n3a, n2}}));
     c.tb.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
     // the wavemaker branch runs on its own stream with its own scratch
     c.tb2 = c.tb;
@@ -860,7 +865,31 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
       if (build_fft_plan(D, c.allocs, &f)) c.tb.fft[c.tb.nfft++] = f;
     }
   }
+  // matrices of the tensor-core passes: F2S in cos and sin and S2F in cos
+  // (what the right-hand side transforms), the S2F of the dealiased grid
+  // also truncated to the free-surface modes
+  c.tb.ntc = 0;
+  if (n2 > 1) {
+    auto add = [&](int D, int form, int sin_kind, double scale, int nout) {
+      for (int i = 0; i < c.tb.ntc; ++i) {
+        const TcMat& m = c.tb.tc[i];
+        if (m.D == D && m.form == form && m.sin_kind == sin_kind && m.scale == scale && nout <= m.nout) return;
+      }
+      if (c.tb.ntc < kTcMats && build_tc_matrix(D, form, sin_kind, scale, nout, c.allocs, &c.tb.tc[c.tb.ntc])) ++c.tb.ntc;
+    };
+    for (int axis = 0; axis < 2; ++axis) {
+      const int n = axis ? n2 : n1, nd = axis ? nd2 : nd1;
+      for (int N : {n, nd}) {
+        add(N - 1, 0, 0, 1.0, N);
+        add(N - 1, 0, 1, 1.0, N);
+        add(N - 1, 0, 0, 2.0 * (1.0 / (N - 1)), N);
+      }
+      if (nd > n) add(nd - 1, 1, 0, 2.0 * (1.0 / (nd - 1)), n);
+    }
+  }
   for (Tables* t : {&c.tb2, &c.tb3}) {
+    t->ntc = c.tb.ntc;
+    for (int i = 0; i < c.tb.ntc; ++i) t->tc[i] = c.tb.tc[i];
     t->q_n1 = d.q_n1; t->q_n2 = d.q_n2; t->q_nd1 = d.q_nd1; t->q_nd2 = d.q_nd2; t->q_add = d.q_add;
     t->nfft = c.tb.nfft;
     for (int i = 0; i < c.tb.nfft; ++i) t->fft[i] = c.tb.fft[i];

@@ -1735,6 +1735,55 @@ void launch_ytl(AxisBatch& b, bool early, cudaStream_t st) {
   });
 }
 
+// FP64 FMAs per line of the sum passes of a job, as its launcher picks them.
+double sum_cost(const AxisJob& J, bool ypass) {
+  const int nin = std::min(J.nin, J.N);
+  int A = 0, B = 0;
+  if (!ypass) {
+    pick_factors(J.D, nin, J.nout, &A, &B);
+    return A > 0 ? x_two_level_cost(A, B, J.D, nin, J.nout) : 0.5 * (double)nin * J.nout;
+  }
+  pick_factors_y(J.D, nin, J.nout, &A, &B);
+  if (A == 0) return 0.5 * (double)nin * J.nout;
+  AxisJob t = J;
+  t.A = A;
+  t.B = B;
+  t.mode = ytl_can_pair(J.D, A, B, J.nout, J.N) ? 1 : 0;
+  return y_two_level_fmas(t);
+}
+
+// Time (us) of a job off the tensor cores, measured on GB300 over 66 to 4100
+// points: 2.2 ps per unit of the FFT plan's cost, 4 ps per FMA of the sums.
+double pass_time(const AxisJob& J, const Tables& tb, bool ypass) {
+  if (!(J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0)) return 0.0;
+  const double sums = sum_cost(J, ypass);
+  const FftPlanInfo* f = fft_choice(J, tb, sums);
+  return (double)J.nlines * (f ? 2.2e-6 * f->cost_line_df : 4e-6 * sums);
+}
+
+// The jobs that run on the tensor cores (tcx.cu) leave the batch.  `next`, if
+// given, are the y jobs that read the outputs of b's x jobs.
+void launch_tensor(AxisBatch& b, const Tables& tb, cudaStream_t st, AxisBatch* next = nullptr) {
+  AxisBatch t{}, rest{};
+  t.njobs = rest.njobs = 0;
+  t.acc = rest.acc = b.acc;
+  int from[kMaxJobs];
+  for (int i = 0; i < b.njobs; ++i) {
+    if (!b.job[i].tc) {
+      rest.job[rest.njobs++] = b.job[i];
+      continue;
+    }
+    from[t.njobs] = i;
+    t.job[t.njobs] = b.job[i];
+    if (next) t.job[t.njobs].cmax = reinterpret_cast<unsigned*>(tb.cs) + (long long)i * (kTcMaxD + 8);
+    ++t.njobs;
+  }
+  if (t.njobs == 0 || !launch_tc_jobs(t, tb, st)) return;
+  b = rest;
+  if (next)
+    for (int i = 0; i < t.njobs; ++i) next->job[from[i]].lmax = t.job[i].cmax;
+}
+
 // y passes: two-level where the length factors well (scratch permitting),
 // direct sums otherwise
 void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
@@ -1742,7 +1791,24 @@ void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
   b.njobs = b2.njobs = bf.njobs = 0;
   b.acc = b2.acc = bf.acc = in.acc;
   const FftPlanInfo* fplan[kMaxJobs];
-  long long cs_used = 0;
+  if (tb.ntc) {
+    // jobs whose x pass did not decide for them: a y pass alone
+    AxisBatch alone{};
+    int from[kMaxJobs];
+    double alt[kMaxJobs];
+    for (int i = 0; i < in.njobs; ++i)
+      if (!in.job[i].tc && !in.job[i].tc_decided) {
+        from[alone.njobs] = i;
+        alt[alone.njobs] = pass_time(in.job[i], tb, true);
+        alone.job[alone.njobs++] = in.job[i];
+      }
+    AxisJob* jobs[1] = {alone.job};
+    const double* alts[1] = {alt};
+    tc_choose(jobs, alts, 1, alone.njobs, tb);
+    for (int i = 0; i < alone.njobs; ++i) in.job[from[i]].tc = alone.job[i].tc;
+  }
+  launch_tensor(in, tb, st);
+  long long cs_used = tb.ntc ? kTcMaxBytes / (long long)sizeof(double) : 0;  // behind the maxima and the flag
   for (int i = 0; i < in.njobs; ++i) {
     AxisJob J = in.job[i];
     J.A = J.B = 0;
@@ -1750,18 +1816,7 @@ void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
     const bool c1s1 = (J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0);
     if (c1s1) {
       const int nin = std::min(J.nin, J.N);
-      int A = 0, B = 0;
-      pick_factors_y(J.D, nin, J.nout, &A, &B);
-      double other = 0.5 * (double)nin * J.nout;
-      if (A > 0) {
-        J.A = A;
-        J.B = B;
-        J.mode = ytl_can_pair(J.D, A, B, J.nout, J.N) ? 1 : 0;
-        other = y_two_level_fmas(J);
-        J.A = J.B = 0;
-        J.mode = 0;
-      }
-      if (const FftPlanInfo* f = fft_choice(J, tb, other)) {
+      if (const FftPlanInfo* f = fft_choice(J, tb, sum_cost(J, true))) {
         fplan[bf.njobs] = f;
         bf.job[bf.njobs++] = J;
         continue;
@@ -1926,7 +1981,20 @@ void launch_ordered(const XfReq* reqs, const int* idx, int n, const Tables& tb, 
   b2.njobs = bd.njobs = bf.njobs = 0;
   b2.acc = bd.acc = bf.acc = bx.acc;
   const FftPlanInfo* fplan[kMaxJobs];
-  long long cs_used = 0;
+  if (tb.ntc && by.njobs == bx.njobs) {
+    AxisJob* jobs[2] = {bx.job, by.job};
+    double altx[kMaxJobs], alty[kMaxJobs];
+    for (int i = 0; i < bx.njobs; ++i) {
+      altx[i] = pass_time(bx.job[i], tb, false);
+      alty[i] = pass_time(by.job[i], tb, true);
+      // a y pass with a matrix whose x pass has none is looked at alone
+      by.job[i].tc_decided = bx.job[i].D == bx.job[i].N - 1;
+    }
+    const double* alts[2] = {altx, alty};
+    tc_choose(jobs, alts, 2, bx.njobs, tb);
+  }
+  launch_tensor(bx, tb, st, by.njobs ? &by : nullptr);
+  long long cs_used = tb.ntc ? kTcMaxBytes / (long long)sizeof(double) : 0;  // behind the maxima and the flag
   for (int i = 0; i < bx.njobs; ++i) {
     AxisJob J = bx.job[i];
     J.A = J.B = 0;
@@ -1934,10 +2002,7 @@ void launch_ordered(const XfReq* reqs, const int* idx, int n, const Tables& tb, 
     const bool c1s1 = (J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0);
     if (c1s1) {
       const int nin = std::min(J.nin, J.N);
-      int A = 0, B = 0;
-      pick_factors(J.D, nin, J.nout, &A, &B);
-      const double other = A > 0 ? x_two_level_cost(A, B, J.D, nin, J.nout) : 0.5 * (double)nin * J.nout;
-      if (const FftPlanInfo* f = fft_choice(J, tb, other)) {
+      if (const FftPlanInfo* f = fft_choice(J, tb, sum_cost(J, false))) {
         fplan[bf.njobs] = f;
         bf.job[bf.njobs++] = J;
         continue;
