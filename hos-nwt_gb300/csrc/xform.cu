@@ -525,290 +525,245 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
 // and twiddles staged in shared memory), then run FMA loops over shared
 // memory: one round trip to L2 per pass instead of a chain of dependent
 // scattered loads.
+//
+// What bounds them on GB300 is FP64 issue: a warp's FP64 instruction holds its
+// scheduler's pipe for 64 cycles, whatever the warps beside it do, so a pass over
+// one line (150k to 250k FMAs, about 6000 warp instructions) takes under a
+// microsecond only when it lies on most of the 608 schedulers.  So both passes cut
+// their sums into parts until the CTAs cover the SMs, keep every FP64 operation that
+// is not an FMA of the sum out of the loops (weights and signs by exponent and
+// sign bits, scales in one product per output), and add the parts up by
+// shuffles.  One line of D = 3074: pass 1 9.5 us -> 4.9, pass 2 5.0 -> 4.0 in the step of
+// the irregular 2-D tank, where the former split used 54 and 33 CTAs.
 constexpr int kP1Threads = 128;
-constexpr int kP2Threads = 128;  // 4 warps split the j2 sum of 32 outputs
+constexpr int kP2Threads = 128;
 constexpr int kP2Warps = kP2Threads / 32;
 
-// Thread-block clusters: a sum too long for one SM is split over the CTAs of
-// a cluster, whose partial results are combined through distributed shared
-// memory by rank 0 in rank order.
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" :::
-                   "memory");
-}
-__device__ __forceinline__ double ld_cluster(const double* local, unsigned rank) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(local);
-  unsigned ra;
-  double v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(ra) : "memory");
-  return v;
-}
-
-// pass 1: cluster = (job, line, group of kpc consecutive k' <= A/2); CTA r
-// of the cluster sums j1 in its slice of [0, K).  The even and odd j1 terms
-// are summed apart: cos / sin(pi j1 (A - k') / A) = +-(-1)^j1 cos / sin(pi
-// j1 k' / A), so the same four sums give C, S at k' and at A - k' and half
-// of the k' are computed.  Threads own (k', part, j2) items with j2
-// fastest: staged inputs are read without bank conflicts and the j1
-// twiddles are broadcast.  Slices hold an even number of j1 (Kc2), so a
-// local index has the parity of its global j1.
 __host__ __device__ inline int p1_half(int A) { return A / 2; }
-__host__ __device__ inline int p1_slice(int K, int ncl) { return (((K + ncl - 1) / ncl) + 1) & ~1; }
+// Pass 1: a CTA takes nk values of k' <= A/2 times G of j2, every sum over j1 in
+// P parts.
+struct P1Shape {
+  int nk, G, kblocks, jblocks;
+};
+__host__ __device__ inline P1Shape p1_shape(int A, int B, int K, int P) {
+  P1Shape s;
+  const int items = kP1Threads / P;
+  // the twiddles of nk values within 96 KB
+  int cap = 96 * 1024 / (16 * (K + 1));
+  if (cap < 1) cap = 1;
+  s.nk = p1_half(A) + 1 < items ? p1_half(A) + 1 : items;
+  if (s.nk > cap) s.nk = cap;
+  s.G = items / s.nk;
+  if (s.G > B) s.G = B;
+  s.kblocks = (p1_half(A) + s.nk) / s.nk;
+  s.jblocks = (B + s.G - 1) / s.G;
+  return s;
+}
 
+// x or -x by the sign bit
+__device__ __forceinline__ double flip_if(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// pass 1: CTA = (job, line, nk values of k', G values of j2).  The even and odd
+// j1 terms are summed apart: cos / sin(pi j1 (A - k') / A) = +-(-1)^j1 cos /
+// sin(pi j1 k' / A), so the same four sums give C, S at k' and at A - k' and
+// half of the k' are computed.  Threads own (k', j2, part) with k' fastest:
+// twiddles are read without bank conflicts, inputs are broadcast.  The inputs
+// enter with the interior weight 1; pass 2 multiplies the outputs by it.
 template <int NJ>
-__global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<NJ> b, int kpc, int ncl) {
+__global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<NJ> b, int P) {
   extern __shared__ double sm1[];
+  __shared__ double red[4 * kP1Threads];
   int jb = 0;
   while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
   const AxisJob& J = b.job[jb];
   const int A = J.A, B = J.B, D = J.D, D4 = 4 * D, H = p1_half(A);
-  const int ngrp = (H + 1 + kpc - 1) / kpc;
-  const int local = (blockIdx.x - b.start[jb]) / ncl;
-  const unsigned rank = ncl > 1 ? cluster_rank() : 0u;
-  const int line = local / ngrp;
-  const int kp0 = (local - line * ngrp) * kpc;
-  const int nkp = min(kpc, H + 1 - kp0);
-  const int j_end = min(J.jhi, J.nin);  // terms j in [jlo, j_end)
-  const int K = (j_end + B - 1) / B;
-  const int Kc = p1_slice(K, ncl);
-  const int ja1 = min(K, (int)rank * Kc), Kl = min(K, ja1 + Kc) - ja1;
-  const int Klp = (Kl + 1) & ~1;    // padded to whole (even, odd) pairs
-  double* fin = sm1;                // kpc * B (C, S, C', S') of this CTA's slice
-  double* xs = fin + 4 * kpc * B;   // Kc * B weighted inputs, zero outside the sum
-  double* tc = xs + Kc * B;         // kpc * Kc cos(pi j1 k' / A)
-  double* ts = tc + kpc * Kc;       // kpc * Kc sin(pi j1 k' / A)
-  double* red = ts + kpc * Kc;      // partial sums of the items
+  const int j_end = min(J.jhi, J.nin), jlo = J.jlo;  // terms j in [jlo, j_end)
+  const int K = (j_end + B - 1) / B, Kp = (K + 1) & ~1;
+  const P1Shape sh = p1_shape(A, B, K, P);
+  int local = blockIdx.x - b.start[jb];
+  const int kb = local % sh.kblocks;
+  local /= sh.kblocks;
+  const int j20 = (local % sh.jblocks) * sh.G, line = local / sh.jblocks;
+  const int kp0 = kb * sh.nk, nk = min(sh.nk, H + 1 - kp0), G = min(sh.G, B - j20);
+  double2* tw = reinterpret_cast<double2*>(sm1);                    // [j1][k'] cos, sin(pi j1 k' / A)
+  double* xs = sm1 + 2 * (size_t)Kp * sh.nk;                        // [j1][j2] inputs, zero outside the sum
   const double* __restrict__ x = J.in + (long long)line * J.in_sl;
   const double* __restrict__ wr = J.win ? J.win + (long long)line * J.win_sl : nullptr;
+  const double* __restrict__ q = J.q;
   auto stage_twiddles = [&]() {
-    for (int t = threadIdx.x; t < nkp * Klp; t += kP1Threads) {
-      const int kpl = t / Klp, jl = t - kpl * Klp;
-      double c = 0.0, sn = 0.0;
-      if (jl < Kl) {
-        // pi j1 k' / A = pi (2 B j1 k') / (2 D); both factors below 4D
-        const unsigned step = (2u * (unsigned)B * (unsigned)(kp0 + kpl)) % (unsigned)D4;
-        const int m = (int)((step * (unsigned)(ja1 + jl)) % (unsigned)D4);
-        c = twiddle(J.q, D, m);
-        sn = twiddle(J.q, D, m >= D ? m - D : m + 3 * D);
-      }
-      tc[kpl * Kc + jl] = c;
-      ts[kpl * Kc + jl] = sn;
+    for (int t = threadIdx.x; t < nk * Kp; t += kP1Threads) {
+      const int j1 = t / nk, kpl = t - j1 * nk;
+      // pi j1 k' / A = pi (2 B j1 k') / (2 D); both factors below 4D
+      const unsigned step = (2u * (unsigned)B * (unsigned)(kp0 + kpl)) % (unsigned)D4;
+      const int m = (int)((step * (unsigned)j1) % (unsigned)D4);
+      tw[t] = make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
     }
   };
   if (b.early) stage_twiddles();
+  const bool half0 = J.w0 != J.wm, halfD = J.wl != J.wm;
+  const int N = J.N;
+  const long long in_sk = J.in_sk, win_sk = J.win_sk;
   pdl_wait();
   if (!b.early) stage_twiddles();
-  for (int t = threadIdx.x; t < Klp * B; t += kP1Threads) {
-    const int j = ja1 * B + t;
+  for (int t = threadIdx.x; t < Kp * G; t += kP1Threads) {
+    const int j1 = t / G, j = j1 * B + j20 + (t - j1 * G);
     double v = 0.0;
-    if (t < Kl * B && j >= J.jlo && j < j_end) {
-      const double w = (j == 0) ? J.w0 : ((j == J.N - 1) ? J.wl : J.wm);
-      v = w * in_at(x, J.in_sk, wr, J.win_sk, j);
+    if (j1 < K && j >= jlo && j < j_end) {
+      v = in_at(x, in_sk, wr, win_sk, j);
+      if ((j == 0 && half0) || (j == N - 1 && halfD)) v *= 0.5;
     }
     xs[t] = v;
   }
   __syncthreads();
-  const int P = max(1, kP1Threads / (nkp * B));  // parts splitting the j1 pair sum
-  const int nitem = nkp * P * B;
-  const int npair = Klp / 2;
-  for (int it = threadIdx.x; it < nitem; it += kP1Threads) {
-    const int j2 = it % B, r = it / B;
-    const int part = r % P, kpl = r / P;
-    const double* tcp = tc + kpl * Kc;
-    const double* tsp = ts + kpl * Kc;
-    double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
-#pragma unroll 2
-    for (int q = part; q < npair; q += P) {
-      const double v0 = xs[(2 * q) * B + j2], v1 = xs[(2 * q + 1) * B + j2];
-      ce = fma(v0, tcp[2 * q], ce);
-      se = fma(v0, tsp[2 * q], se);
-      co = fma(v1, tcp[2 * q + 1], co);
-      so = fma(v1, tsp[2 * q + 1], so);
+  const int items = nk * G;
+  const int r = threadIdx.x / nk, kpl = threadIdx.x - r * nk;
+  const int part = r / G, j2l = r - part * G;
+  double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
+  if (part < P) {
+#pragma unroll 4
+    for (int p = part; p < Kp / 2; p += P) {
+      const double v0 = xs[2 * p * G + j2l], v1 = xs[(2 * p + 1) * G + j2l];
+      const double2 t0 = tw[2 * p * nk + kpl], t1 = tw[(2 * p + 1) * nk + kpl];
+      ce = fma(v0, t0.x, ce);
+      se = fma(v0, t0.y, se);
+      co = fma(v1, t1.x, co);
+      so = fma(v1, t1.y, so);
     }
-    red[4 * it] = ce + co;      // C(k')
-    red[4 * it + 1] = se + so;  // S(k')
-    red[4 * it + 2] = ce - co;  // C(A - k')
-    red[4 * it + 3] = so - se;  // S(A - k')
+    double* rp = red + part * 4 * items + 4 * (j2l * nk + kpl);
+    rp[0] = ce;
+    rp[1] = se;
+    rp[2] = co;
+    rp[3] = so;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < nkp * B; t += kP1Threads) {
-    const int j2 = t % B, kpl = t / B;
-    double f[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int part = 0; part < P; ++part) {
-      const int it = (kpl * P + part) * B + j2;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) f[u] += red[4 * it + u];
+  // the parts' sums: R threads per value, then the folds between values v and
+  // v ^ 2 of an item, by shuffles
+  const int R = P >= 16 ? 4 : (P >= 8 ? 2 : 1);
+  double* cs = J.cs + ((long long)line * B + j20) * (A + 1) * 2;
+  for (int t0 = 0; t0 < 4 * items * R; t0 += kP1Threads) {
+    const int t = t0 + threadIdx.x, iv = t / R;
+    const bool on = iv < 4 * items;
+    double f = 0.0;
+    if (on) {
+      f = red[(t % R) * 4 * items + iv];
+      for (int p = t % R + R; p < P; p += R) f += red[p * 4 * items + iv];
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) fin[4 * t + u] = f[u];
-  }
-  if (ncl > 1) cluster_sync_all();
-  else __syncthreads();
-  if (rank == 0) {
-    for (int t = threadIdx.x; t < nkp * B; t += kP1Threads) {
-      double f[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) f[u] = fin[4 * t + u];
-      for (int r = 1; r < ncl; ++r)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) f[u] += ld_cluster(fin + 4 * t + u, (unsigned)r);
-      const int j2 = t % B, kp = kp0 + t / B;
-      double* cs = J.cs + (((long long)line * B + j2) * (A + 1)) * 2;
-      cs[2 * kp] = f[0];
-      cs[2 * kp + 1] = f[1];
-      if (A - kp != kp) {
-        cs[2 * (A - kp)] = f[2];
-        cs[2 * (A - kp) + 1] = f[3];
-      }
+    if (R > 1) f += __shfl_xor_sync(0xffffffffu, f, 1);
+    if (R > 2) f += __shfl_xor_sync(0xffffffffu, f, 2);
+    const double o = __shfl_xor_sync(0xffffffffu, f, 2 * R);
+    const int v = iv & 3;
+    // C(k') = ce + co, S(k') = se + so, C(A - k') = ce - co, S(A - k') = so - se
+    const double y = flip_if(f, v == 2) + flip_if(o, v == 3);
+    if (on && t % R == 0) {
+      const int it = iv >> 2, kp = kp0 + it % nk;
+      double* c = cs + (long long)(it / nk) * (A + 1) * 2;
+      if (v < 2) c[2 * kp + v] = y;
+      else if (A - kp != kp) c[2 * (A - kp) + v - 2] = y;
     }
   }
-  if (ncl > 1) cluster_sync_all();  // remote reads done before any CTA exits
 }
 
-// pass 2: cluster = (job, line, 32 outputs); CTA r of the cluster sums j2 in
-// its slice of [0, B).  The slice's twiddles cos/sin(pi j2 k / D) are staged
-// first; lanes own outputs (their C, S loads are contiguous), warps split
-// the slice and are combined in a fixed order.
-//
 // Paired jobs (mode 1: B even, every output wanted): with B even, (-1)^j =
 // (-1)^j2, so y(D - k) = +-sum_j2 (-1)^j2 T_j2(k) for the terms T_j2(k) of
-// y(k).  Lanes own k <= D/2; warps (and cluster slices, of even length)
-// hold j2 of one parity, and the even and odd sums E, O give y(k) = E + O
-// and y(D - k) = E - O (cos kind) or O - E (sin kind).
-__host__ __device__ inline int p2_slice(int B, int ncl, bool paired) {
-  const int c = (B + ncl - 1) / ncl;
-  return (paired && ncl > 1) ? ((c + 1) & ~1) : c;
-}
+// y(k).  Lanes own k <= D/2, and the sums E, O over even and odd j2 give y(k)
+// = E + O and y(D - k) = E - O (cos kind) or O - E (sin kind).
 __host__ __device__ inline int p2_lanes(const AxisJob& J) { return J.mode == 1 ? J.D / 2 + 1 : J.nout; }
 
-__device__ __forceinline__ void p2_put(const AxisJob& J, const AccEpi& acc, int line, int k, double y) {
+// scale of output k; w: the interior weight, where pass 1 left it out
+__device__ __forceinline__ double p2_scale(const AxisJob& J, int k, double w) {
+  return ((k == 0) ? J.s0 : ((k == J.N - 1) ? J.sl : J.sm)) * J.gscale * w;
+}
+__device__ __forceinline__ void p2_put(const AxisJob& J, const AccEpi& acc, int line, int k, double y, double scale) {
   if (k >= J.nout) return;
   const bool on = k >= J.klo && k < J.khi;
   const long long e = (long long)line * J.out_sl + (long long)k * J.out_sk;
-  const double sc = (k == 0) ? J.s0 : ((k == J.N - 1) ? J.sl : J.sm);
-  const double v = on ? y * sc * J.gscale : 0.0;
+  const double v = on ? y * scale : 0.0;
   J.out[e] = v;
   if (J.epi) acc_epilogue(acc, e, v);
 }
 
-template <int NJ>
-__global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<NJ> b, int ncl) {
+// pass 2: CTA = (job, line, KO outputs).  A warp holds KO outputs times 32 / KO
+// slices of the j2 sum, warp w the slices w, w + 4, ...: every slice of a warp
+// has the parity of w (paired jobs), its slices meet by shuffles and the four
+// warps in shared memory.
+template <int NJ, int KO>
+__global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<NJ> b) {
   extern __shared__ double sm2[];
-  __shared__ double red[kP2Warps][32];
-  __shared__ double fin[2][32];
+  __shared__ double red[kP2Warps][KO];
+  constexpr int SL = kP2Warps * (32 / KO);
   int jb = 0;
   while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
   const AxisJob& J = b.job[jb];
   const int A = J.A, B = J.B, D = J.D, D4 = 4 * D;
   const bool paired = J.mode == 1;
   const int nlane = p2_lanes(J);
-  const int nkb = (nlane + 31) / 32;
-  const int local = (blockIdx.x - b.start[jb]) / ncl;
-  const unsigned rank = ncl > 1 ? cluster_rank() : 0u;
+  const int nkb = (nlane + KO - 1) / KO;
+  const int local = blockIdx.x - b.start[jb];
   const int line = local / nkb;
-  const int k0 = (local - line * nkb) * 32;
-  const int Bc = p2_slice(B, ncl, paired);
-  const int ja2 = min(B, (int)rank * Bc), Bl = min(B, ja2 + Bc) - ja2;
+  const int k0 = (local - line * nkb) * KO;
+  const double* __restrict__ q = J.q;
+  double2* tw = reinterpret_cast<double2*>(sm2);  // [j2][k] cos, sin(pi j2 k / D)
   auto stage_twiddles = [&]() {
-    for (int t = threadIdx.x; t < Bl * 32; t += kP2Threads) {
-      const int j2 = ja2 + (t >> 5), k = k0 + (t & 31);
-      // pi j2 k / D; j2 < D and k < N, so 2 j2 k fits in 32 bits for N < 32768
+    for (int t = threadIdx.x; t < B * KO; t += kP2Threads) {
+      const int j2 = t / KO, k = k0 + (t % KO);
+      // j2 < D and k < N, so 2 j2 k fits in 32 bits for N < 32768
       const int m = (int)((2u * (unsigned)j2 * (unsigned)k) % (unsigned)D4);
-      sm2[2 * t] = twiddle(J.q, D, m);
-      sm2[2 * t + 1] = twiddle(J.q, D, m >= D ? m - D : m + 3 * D);
+      tw[t] = make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
     }
   };
   if (b.early) stage_twiddles();
-  pdl_wait();
-  if (!b.early) stage_twiddles();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = k0 + lane;
+  const int kl = lane % KO, slice = warp + kP2Warps * (lane / KO);
+  const int k = k0 + kl;
   const bool on = paired ? k < nlane : (k < J.nout && k >= J.klo && k < J.khi);
   int kp = k % (2 * A);
-  double ssign = 1.0;
-  if (kp > A) {
-    kp = 2 * A - kp;
-    ssign = -1.0;
-  }
+  const bool sneg = kp > A;
+  if (sneg) kp = 2 * A - kp;
   const bool is_sin = (J.off != 0);
-  const double* cs = J.cs + ((long long)line * B * (A + 1) + kp) * 2;
-  // C, S of this lane's j2 terms, loaded before the twiddles are needed
-  constexpr int kMaxOwn = 16;
-  double Cv[kMaxOwn], Sv[kMaxOwn];
-  const int nown = on ? min(kMaxOwn, (Bl - warp + kP2Warps - 1) / kP2Warps) : 0;
-#pragma unroll
-  for (int i = 0; i < kMaxOwn; ++i) {
-    if (i < nown) {
-      const long long o = (long long)(ja2 + warp + i * kP2Warps) * (A + 1) * 2;
-      Cv[i] = __ldcg(cs + o);
-      Sv[i] = __ldcg(cs + o + 1);
-    }
-  }
-  __syncthreads();
+  const double2* cs = reinterpret_cast<const double2*>(J.cs) + (long long)line * B * (A + 1) + kp;
+  const double sck = p2_scale(J, k, J.wm), scm = p2_scale(J, D - k, J.wm);
+  pdl_wait();
+  if (!b.early) stage_twiddles();
+  // cos kind: cw C - sw S; sin kind: sw C + cw S (S with the sign of its fold)
+  const bool neg = sneg != !is_sin;
+  constexpr int kOwn = 8;  // terms in flight
   double acc = 0.0;
+  double2 v[kOwn];
+  auto load = [&](int j2) {
 #pragma unroll
-  for (int i = 0; i < kMaxOwn; ++i) {
-    if (i < nown) {
-      const int t = warp + i * kP2Warps;  // j2 - ja2
-      const double cw = sm2[2 * (t * 32 + lane)], sw = sm2[2 * (t * 32 + lane) + 1];
-      const double S = ssign * Sv[i];
-      if (is_sin) acc = fma(cw, S, fma(sw, Cv[i], acc));
-      else acc = fma(cw, Cv[i], fma(-sw, S, acc));
-    }
-  }
-  // j2 beyond the register-held terms
-  if (on) {
-    for (int t = warp + kMaxOwn * kP2Warps; t < Bl; t += kP2Warps) {
-      const long long o = (long long)(ja2 + t) * (A + 1) * 2;
-      const double cw = sm2[2 * (t * 32 + lane)], sw = sm2[2 * (t * 32 + lane) + 1];
-      const double C = __ldcg(cs + o), S = ssign * __ldcg(cs + o + 1);
-      if (is_sin) acc = fma(cw, S, fma(sw, C, acc));
-      else acc = fma(cw, C, fma(-sw, S, acc));
-    }
-  }
-  red[warp][lane] = acc;
+    for (int i = 0; i < kOwn; ++i)
+      if (on && j2 + i * SL < B) v[i] = __ldcg(cs + (long long)(j2 + i * SL) * (A + 1));
+  };
+  load(slice);
   __syncthreads();
-  if (warp == 0) {
-    if (paired) {
-      // warps of even index hold even j2 (kP2Warps and ja2 are even)
-      double e = 0.0, o = 0.0;
+  for (int j2 = slice; j2 < B; j2 += kOwn * SL) {
+    if (j2 != slice) load(j2);
 #pragma unroll
-      for (int w = 0; w < kP2Warps; w += 2) {
-        e += red[w][lane];
-        o += red[w + 1][lane];
+    for (int i = 0; i < kOwn; ++i) {
+      if (on && j2 + i * SL < B) {
+        const double2 t = tw[(j2 + i * SL) * KO + kl];
+        acc = fma(is_sin ? t.y : t.x, v[i].x, acc);
+        acc = fma(flip_if(is_sin ? t.x : t.y, neg), v[i].y, acc);
       }
-      fin[0][lane] = e;
-      fin[1][lane] = o;
-    } else {
-      double y = 0.0;
-#pragma unroll
-      for (int w = 0; w < kP2Warps; ++w) y += red[w][lane];
-      fin[0][lane] = y;
     }
   }
-  if (ncl > 1) cluster_sync_all();
-  else __syncthreads();
-  if (rank == 0 && warp == 0) {
-    double y = fin[0][lane];
-    for (int r = 1; r < ncl; ++r) y += ld_cluster(&fin[0][lane], (unsigned)r);
+#pragma unroll
+  for (int off = KO; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (lane < KO) red[warp][lane] = acc;
+  __syncthreads();
+  if (threadIdx.x < KO) {
+    const double e = red[0][lane] + red[2][lane], o = red[1][lane] + red[3][lane];
     if (paired) {
-      double o = fin[1][lane];
-      for (int r = 1; r < ncl; ++r) o += ld_cluster(&fin[1][lane], (unsigned)r);
       if (k < nlane) {
-        p2_put(J, b.acc, line, k, y + o);
-        if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? o - y : y - o);
+        p2_put(J, b.acc, line, k, e + o, sck);
+        if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? o - e : e - o, scm);
       }
     } else if (k < J.nout) {
-      p2_put(J, b.acc, line, k, on ? y : 0.0);
+      p2_put(J, b.acc, line, k, on ? e + o : 0.0, sck);
     }
   }
-  if (ncl > 1) cluster_sync_all();  // remote reads done before any CTA exits
 }
 
 // pass 2 for launches with many lines (the x passes of 3-D tanks):
@@ -873,11 +828,11 @@ __global__ void __launch_bounds__(kP2Threads) two_level_pass2_lines(const AxisBa
     }
     if (paired) {
       if (k < nlane) {
-        p2_put(J, b.acc, line, k, ae + ao);
-        if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? ao - ae : ae - ao);
+        p2_put(J, b.acc, line, k, ae + ao, p2_scale(J, k, J.wm));
+        if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? ao - ae : ae - ao, p2_scale(J, D - k, J.wm));
       }
     } else {
-      p2_put(J, b.acc, line, k, on ? ae : 0.0);
+      p2_put(J, b.acc, line, k, on ? ae : 0.0, p2_scale(J, k, J.wm));
     }
   }
 }
@@ -1070,10 +1025,10 @@ __global__ void __launch_bounds__(kFThreads) two_level_fused(const AxisBatchT<NJ
     const int s = t * nsplit + u;
     const int k = 2 * A * (s / nr) + fused_residue(A, g, s % nr);
     if (paired) {
-      p2_put(J, b.acc, line, k, e + o);
-      if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? o - e : e - o);
+      p2_put(J, b.acc, line, k, e + o, p2_scale(J, k, 1.0));
+      if (D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? o - e : e - o, p2_scale(J, D - k, 1.0));
     } else {
-      p2_put(J, b.acc, line, k, e + o);
+      p2_put(J, b.acc, line, k, e + o, p2_scale(J, k, 1.0));
     }
   }
 }
@@ -1406,30 +1361,14 @@ void allow_smem(K kern) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
-// Shared memory of pass 1 for a job with kpc values of k' per cluster and
-// ncl CTAs per cluster, and of pass 2 with ncl CTAs per cluster.
-size_t pass1_smem(const AxisJob& J, int kpc, int ncl) {
-  const int j_end = std::min(J.jhi, J.nin);
-  const int K = (j_end + J.B - 1) / J.B;
-  const int Kc = p1_slice(K, ncl);
-  const int nkp = std::min(kpc, p1_half(J.A) + 1);
-  const int items = std::max(kP1Threads, nkp * J.B);
-  return sizeof(double) *
-         (4 * (size_t)kpc * J.B + (size_t)Kc * J.B + 2 * (size_t)kpc * Kc + 4 * (size_t)items);
+int p1_terms(const AxisJob& J) { return (std::min(J.jhi, J.nin) + J.B - 1) / J.B; }
+// Shared memory of the passes (the twiddles, pass 1 also the inputs).
+size_t pass1_smem(const AxisJob& J, int P) {
+  const int K = p1_terms(J), Kp = (K + 1) & ~1;
+  const P1Shape s = p1_shape(J.A, J.B, K, P);
+  return sizeof(double) * ((size_t)Kp * s.nk * 2 + (size_t)Kp * s.G);
 }
-size_t pass2_smem(const AxisJob& J, int ncl) {
-  return sizeof(double) * 2 * 32 * (size_t)p2_slice(J.B, ncl, J.mode == 1);
-}
-
-// Cluster size: split a CTA's sum only while its FP64 work (`fmas`, at about
-// 2 FMAs per cycle per SM) exceeds the cost of the cluster barriers, the
-// launch has room on the SMs, and each CTA keeps at least 4 terms.
-int pick_cluster(long long units, long long fmas, int terms, int nsm) {
-  int ncl = 1;
-  while (ncl < 8 && fmas / ncl > 4096 && units * ncl < 4LL * std::max(nsm, 1) && 2 * ncl * 4 <= terms)
-    ncl *= 2;
-  return ncl;
-}
+size_t pass2_smem(const AxisJob& J, int KO) { return sizeof(double) * 2 * KO * (size_t)J.B; }
 
 // FMAs of a two-level pass pair on one line
 double two_level_fmas(const AxisJob& J) {
@@ -1453,42 +1392,41 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   attr_set.run([&] {
     for (int nj : {1, 2, 4, 8, kMaxJobs})
       with_capacity(nj, [&](auto c) {
-        allow_smem(two_level_pass1<decltype(c)::value>);
-        allow_smem(two_level_pass2<decltype(c)::value>);
+        constexpr int NJ = decltype(c)::value;
+        allow_smem(two_level_pass1<NJ>);
+        allow_smem(two_level_pass2<NJ, 8>);
+        allow_smem(two_level_pass2<NJ, 16>);
+        allow_smem(two_level_pass2<NJ, 32>);
       });
   });
-  // pass 1: one k' per cluster while that gives fewer than two clusters per
-  // SM, else up to 8 k' per cluster so that each CTA reuses its staged row;
-  // the j1 sums are split over a cluster when there are few rows
-  long long rows = 0, kbmax = 0;
-  int kmin = 1 << 30;
-  for (int i = 0; i < b.njobs; ++i) {
-    const AxisJob& J = b.job[i];
-    rows += (long long)J.nlines * (p1_half(J.A) + 1);
-    const int K = (std::min(J.jhi, J.nin) + J.B - 1) / J.B;
-    kmin = std::min(kmin, K);
-    kbmax = std::max(kbmax, (long long)K * J.B);
-  }
-  int kpc = (int)std::min<long long>(8, std::max<long long>(1, rows / (2LL * std::max(nsm, 1))));
-  const int ncl1 = pick_cluster((rows + kpc - 1) / kpc, 2 * kbmax * kpc, kmin, nsm);
+  // pass 1: as many parts per sum as keep the launch within two CTAs per SM
+  // (each part costs its share of the final sums: 16 of them make the FP64
+  // work of one line 1.4 times that of four)
+  auto ctas1 = [&](int P) {
+    long long n = 0;
+    for (int i = 0; i < b.njobs; ++i) {
+      const AxisJob& J = b.job[i];
+      const P1Shape s = p1_shape(J.A, J.B, p1_terms(J), P);
+      n += (long long)J.nlines * s.kblocks * s.jblocks;
+    }
+    return n;
+  };
+  int P = 16;
+  while (P > 2 && ctas1(P) > 2LL * std::max(nsm, 1)) P /= 2;
   size_t smem1 = 0, smem2 = 0;
-  for (int i = 0; i < b.njobs; ++i) smem1 = std::max(smem1, pass1_smem(b.job[i], kpc, ncl1));
-  while (kpc > 1 && smem1 > 160 * 1024) {
-    kpc /= 2;
-    smem1 = 0;
-    for (int i = 0; i < b.njobs; ++i) smem1 = std::max(smem1, pass1_smem(b.job[i], kpc, ncl1));
-  }
   int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
+    const AxisJob& J = b.job[i];
+    const P1Shape s = p1_shape(J.A, J.B, p1_terms(J), P);
+    smem1 = std::max(smem1, pass1_smem(J, P));
     b.start[i] = total;
-    total += b.job[i].nlines * ((p1_half(b.job[i].A) + 1 + kpc - 1) / kpc) * ncl1;
+    total += J.nlines * s.kblocks * s.jblocks;
   }
   b.start[b.njobs] = total;
   if (total > 0)
     with_capacity(b.njobs, [&](auto c) {
       constexpr int NJ = decltype(c)::value;
-      launch_pdl_cluster(two_level_pass1<NJ>, dim3(total), dim3(kP1Threads), smem1, ncl1, st, shrink<NJ>(b),
-                         kpc, ncl1);
+      launch_pdl(two_level_pass1<NJ>, dim3(total), dim3(kP1Threads), smem1, st, shrink<NJ>(b), P);
     });
   // pass 2 with many lines per job: line groups share their staged twiddles
   int minl = 1 << 30;
@@ -1506,7 +1444,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     for (int i = 0; i < b.njobs; ++i) {
       b.start[i] = total;
       total += ((b.job[i].nlines + lpc - 1) / lpc) * ((p2_lanes(b.job[i]) + 31) / 32);
-      smem2 = std::max(smem2, pass2_smem(b.job[i], 1));
+      smem2 = std::max(smem2, pass2_smem(b.job[i], 32));
     }
     b.start[b.njobs] = total;
     with_capacity(b.njobs, [&](auto c) {
@@ -1515,28 +1453,27 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     });
     return;
   }
-  // pass 2: 32 outputs per cluster, the j2 sums split over a cluster when
-  // there are few output blocks
-  long long blocks = 0;
-  int bmin = 1 << 30, bmax = 0;
-  for (int i = 0; i < b.njobs; ++i) {
-    blocks += (long long)b.job[i].nlines * ((p2_lanes(b.job[i]) + 31) / 32);
-    bmin = std::min(bmin, b.job[i].B);
-    bmax = std::max(bmax, b.job[i].B);
-  }
-  const int ncl2 = pick_cluster(blocks, 64LL * bmax, bmin, nsm);
+  // pass 2: fewer outputs per CTA until the launch covers the SMs
+  auto ctas2 = [&](int KO) {
+    long long n = 0;
+    for (int i = 0; i < b.njobs; ++i) n += (long long)b.job[i].nlines * ((p2_lanes(b.job[i]) + KO - 1) / KO);
+    return n;
+  };
+  int KO = 32;
+  while (KO > 8 && ctas2(KO) < std::max(nsm, 1)) KO /= 2;
   total = 0;
   for (int i = 0; i < b.njobs; ++i) {
     b.start[i] = total;
-    total += b.job[i].nlines * ((p2_lanes(b.job[i]) + 31) / 32) * ncl2;
-    smem2 = std::max(smem2, pass2_smem(b.job[i], ncl2));
+    total += b.job[i].nlines * ((p2_lanes(b.job[i]) + KO - 1) / KO);
+    smem2 = std::max(smem2, pass2_smem(b.job[i], KO));
   }
   b.start[b.njobs] = total;
   if (total > 0)
     with_capacity(b.njobs, [&](auto c) {
       constexpr int NJ = decltype(c)::value;
-      launch_pdl_cluster(two_level_pass2<NJ>, dim3(total), dim3(kP2Threads), smem2, ncl2, st, shrink<NJ>(b),
-                         ncl2);
+      if (KO == 8) launch_pdl(two_level_pass2<NJ, 8>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
+      else if (KO == 16) launch_pdl(two_level_pass2<NJ, 16>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
+      else launch_pdl(two_level_pass2<NJ, 32>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
     });
 }
 
