@@ -227,10 +227,15 @@ void launch_transforms(const XfReq* reqs, int nreq, const Tables& tb, double* co
                        cudaStream_t st);
 
 struct Tables;
-// F2S along y only (FOURIER_2_SPACE_y, fourier_FFTW.f90:340-428) of nlines
-// lines that are contiguous in memory; cs: 0 cos, 1 sin.
-void launch_y_f2s(const Tables& tb, const double* in, int nlines, long long y_stride, double* out,
-                  long long out_y_stride, int cs, cudaStream_t st);
+// F2S along y only (FOURIER_2_SPACE_y, fourier_FFTW.f90:340-428) of fields of
+// nlines lines that are contiguous in memory, all in one launch; cs: 0 cos, 1 sin.
+struct YReq {
+  const double* in;
+  double* out;
+  int cs;
+};
+void launch_y_f2s(const Tables& tb, const std::vector<YReq>& reqs, int nlines, long long y_stride,
+                  long long out_y_stride, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // FFT-based passes (fft.cu).  A REDFT00 / RODFT00 pass of length N = D + 1

@@ -64,6 +64,31 @@ __device__ double block_reduce(double v) {
   return v;  // valid in thread 0
 }
 
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// maxima of two values over the block, valid in thread 0
+__device__ void block_max2(unsigned long long& a, unsigned long long& b, unsigned long long (*sh)[32]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  a = warp_max(a);
+  b = warp_max(b);
+  __syncthreads();
+  if (lane == 0) {
+    sh[0][w] = a;
+    sh[1][w] = b;
+  }
+  __syncthreads();
+  if (w == 0) {
+    a = warp_max(lane < nw ? sh[0][lane] : 0ULL);
+    b = warp_max(lane < nw ? sh[1][lane] : 0ULL);
+  }
+}
+
 // returns true in thread 0 of the last block to finish
 __device__ bool last_block(unsigned int* counter) {
   __shared__ bool amlast;
@@ -75,6 +100,15 @@ __device__ bool last_block(unsigned int* counter) {
   }
   __syncthreads();
   return amlast;
+}
+
+// Sum of n partial sums by the whole block, valid in thread 0.  (One thread
+// reading them in turn took 0.2 us per sum batch of four: 100 us of k_gtof's
+// 114 us on the 2061 blocks of a 513 x 257 tank.)
+__device__ double sum_parts(const double* part, int n) {
+  double v = 0.0;
+  for (int b = threadIdx.x; b < n; b += blockDim.x) v += __ldcg(part + b);
+  return block_reduce<0>(v);
 }
 
 __device__ void volume_fix(double* etam, double S, const double* sc, int igeom, double d_hinge,
@@ -122,11 +156,12 @@ __global__ void k_gtof(const double* __restrict__ G1, const double* __restrict__
   }
   const double bs = block_reduce<0>(e);
   if (threadIdx.x == 0) part[blockIdx.x] = bs;
-  if (last_block(counter) && threadIdx.x == 0) {
-    double S = 0.0;
-    for (unsigned int b = 0; b < gridDim.x; ++b) S += __ldcg(part + b);
-    volume_fix(etam, S, sc, igeom, d_hinge, xlen);
-    *counter = 0;
+  if (last_block(counter)) {
+    const double S = sum_parts(part, (int)gridDim.x);
+    if (threadIdx.x == 0) {
+      volume_fix(etam, S, sc, igeom, d_hinge, xlen);
+      *counter = 0;
+    }
   }
 }
 
@@ -134,8 +169,19 @@ __global__ void k_gtof(const double* __restrict__ G1, const double* __restrict__
 // e_{j+1} = e_j / (j+1) * e_1 for j = j0 .. j1-1 (resol_HOS.f90:979-987)
 struct PowArgs {
   double* e[16];
+  double inv[16];  // 1 / (j + 1) rounded
   int j0, j1;
 };
+// v / d from r = 1 / d rounded: q = v r, corrected by its exact remainder
+// (Markstein, 1990): three operations in place of a division's dozen, which at
+// 64 issue cycles each held the steep tank's k_pow_run at 895 us a call.  A v
+// whose remainder could underflow, or that is not finite, is divided.
+__device__ __forceinline__ double div_by(double v, double d, double r) {
+  const int e = (__double2hiint(v) >> 20) & 0x7ff;
+  if (e < 64 || e == 0x7ff) return v / d;
+  const double q = v * r;
+  return fma(fma(-d, q, v), r, q);
+}
 __global__ void k_pow_run(PowArgs a, long long n) {
   pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -143,7 +189,7 @@ __global__ void k_pow_run(PowArgs a, long long n) {
   const double e1 = a.e[0][i];
   double v = a.e[a.j0 - 1][i];
   for (int j = a.j0; j < a.j1; ++j) {
-    v = v / (double)(j + 1) * e1;
+    v = div_by(v, (double)(j + 1), a.inv[j]) * e1;
     a.e[j][i] = v;
   }
 }
@@ -154,12 +200,16 @@ __global__ void k_pow_run(PowArgs a, long long n) {
 // Optionally also the outer sums oscale * (sum of the groups q with
 // outer_of[q] == u), u < nouter: the geta2phiz2 sums of groups that are
 // not dealiased themselves, in the order of k_sum_fields.
+// The terms come sorted by group (stable), so that one sum is live at a time:
+// a predicated add per group and term cost sixteen FP64 issues of which one did
+// work.
 struct GroupTerms {
   const double* x[48];
   const double* y[48];
   double s[48];
   int group[48];
   int nterm;
+  int start[17];  // terms of group g: start[g] .. start[g + 1] - 1
   double* out[16];
   int ngroup;
   int outer_of[16];
@@ -171,27 +221,19 @@ __global__ void k_group_products(GroupTerms g, long long n) {
   pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double acc[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) acc[q] = 0.0;
-  for (int t = 0; t < g.nterm; ++t) {
-    const double v = (g.s[t] * g.x[t][i]) * g.y[t][i];
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (q == g.group[t]) acc[q] += v;
+  double os[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int q = 0; q < g.ngroup; ++q) {
+    double acc = 0.0;
+#pragma unroll 4
+    for (int t = g.start[q]; t < g.start[q + 1]; ++t) acc += (g.s[t] * g.x[t][i]) * g.y[t][i];
+    g.out[q][i] = acc;
+    const int u = g.outer_of[q];
+    if (u == 0) os[0] += acc;
+    else if (u == 1) os[1] += acc;
+    else if (u == 2) os[2] += acc;
+    else if (u == 3) os[3] += acc;
   }
-#pragma unroll
-  for (int q = 0; q < 16; ++q)
-    if (q < g.ngroup) g.out[q][i] = acc[q];
   if (g.nouter > 0) {
-    double os[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      if (q >= g.ngroup) break;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u == g.outer_of[q]) os[u] += acc[q];
-    }
     const double sc = g.oscale[i];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -413,8 +455,9 @@ __device__ void ramp_law(const RampP& r, double time, double* a, double* at, dou
 __global__ void k_eiwt(const double* __restrict__ freq, double* sc, double* eiwt, int nf, RampP rp) {
   pdl_wait();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n == 0) {
-    // the wavemaker law of this stage (single writer of the ramp slots)
+  if (n == 32) {
+    // the wavemaker law of this stage (single writer of the ramp slots), beside
+    // the warp that has the first frequencies
     double a = sc[SC_ALPHA], at = sc[SC_ALPHAT], att = sc[SC_ALPHATT];
     ramp_law(rp, sc[SC_TIME], &a, &at, &att);
     sc[SC_ALPHA] = a;
@@ -981,31 +1024,73 @@ __global__ void k_phiadd_q(const double* __restrict__ a1, const double* __restri
   Qp[o] = a * csh[o];
 }
 
-// phiadd_SL (3-D): contraction over i3 at z = eta of the y-transformed B_q
-__global__ void k_phiadd_contract(const double* __restrict__ eta, const double* __restrict__ kx_add,
-                                  const double* __restrict__ Bt, const double* __restrict__ Bx,
-                                  const double* __restrict__ By, const double* __restrict__ Bz,
-                                  const double* __restrict__ Bp, int n1, int n2, int n3a,
-                                  double* phix, double* phiy, double* phiz, double* phit, double* phi) {
+// phiadd_SL (3-D): contraction over i3 at z = eta of the y-transformed B_q.
+// kx_add(i3) = (2 i3 + 1) pi / 4: cos / sin(kx_add(i3) (eta + 1)) by rotations
+// of 2 phi, phi = pi (eta + 1) / 4, from one sincos per kRestart modes, as in the
+// 1-D tank (a sincos per mode and point held the FP64 pipe for 546 us a call on
+// a 513 x 257 tank; its own error, the rounding of an angle of up to 100, is what
+// the rotations accumulate).  CY threads share the modes of a point where the
+// points alone are too few for the SMs.
+constexpr int kRestart = 32;
+template <int CY>
+__global__ void __launch_bounds__(128) k_phiadd_contract(
+    const double* __restrict__ eta, const double* __restrict__ kx_add, const double* __restrict__ Bt,
+    const double* __restrict__ Bx, const double* __restrict__ By, const double* __restrict__ Bz,
+    const double* __restrict__ Bp, int n1, int n2, int n3a, double* phix, double* phiy, double* phiz, double* phit,
+    double* phi) {
+  constexpr int CX = 128 / CY;
+  __shared__ double r[CY > 1 ? 5 : 1][CY][CX];
   pdl_wait();
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)n1 * n2) return;
-  const int i1 = (int)(i % n1), i2 = (int)(i / n1);
-  const double e1 = eta[i] + 1.0;
+  const int tx = threadIdx.x % CX, ty = threadIdx.x / CX;
+  const long long i = blockIdx.x * (long long)CX + tx;
+  const bool on = i < (long long)n1 * n2;
   double st = 0.0, sx = 0.0, sy = 0.0, sz = 0.0, sp = 0.0;
-  for (int i3 = 0; i3 < n3a; ++i3) {
-    double s, c;
-    sincos(kx_add[i3] * e1, &s, &c);
-    const long long o = i1 + (long long)n1 * i3 + (long long)n1 * n3a * i2;
-    st += c * Bt[o];
-    sx -= c * Bx[o];
-    sy -= c * By[o];
-    sz -= s * Bz[o];
-    sp += c * Bp[o];
+  if (on) {
+    const int i1 = (int)(i % n1), i2 = (int)(i / n1);
+    const double e1 = eta[i] + 1.0;
+    const int ch = (n3a + CY - 1) / CY;
+    const int a = ty * ch, b = min(n3a, a + ch);
+    const long long base = i1 + (long long)n1 * n3a * i2;
+    double s2, c2;
+    sincos(2.0 * kx_add[0] * e1, &s2, &c2);
+    for (int g = a; g < b; g += kRestart) {
+      double s, c;
+      sincos(kx_add[g] * e1, &s, &c);
+      const int ge = min(b, g + kRestart);
+#pragma unroll 4
+      for (int i3 = g; i3 < ge; ++i3) {
+        const long long o = base + (long long)n1 * i3;
+        st = fma(c, __ldg(Bt + o), st);
+        sx = fma(c, __ldg(Bx + o), sx);
+        sy = fma(c, __ldg(By + o), sy);
+        sz = fma(s, __ldg(Bz + o), sz);
+        sp = fma(c, __ldg(Bp + o), sp);
+        const double cn = c * c2 - s * s2;
+        s = s * c2 + c * s2;
+        c = cn;
+      }
+    }
   }
-  phix[i] = sx;
-  phiy[i] = sy;
-  phiz[i] = sz;
+  if constexpr (CY > 1) {
+    r[0][ty][tx] = st;
+    r[1][ty][tx] = sx;
+    r[2][ty][tx] = sy;
+    r[3][ty][tx] = sz;
+    r[4][ty][tx] = sp;
+    __syncthreads();
+    if (ty != 0) return;
+    for (int q = 1; q < CY; ++q) {
+      st += r[0][q][tx];
+      sx += r[1][q][tx];
+      sy += r[2][q][tx];
+      sz += r[3][q][tx];
+      sp += r[4][q][tx];
+    }
+  }
+  if (!on) return;
+  phix[i] = -sx;
+  phiy[i] = -sy;
+  phiz[i] = -sz;
   phit[i] = st;
   phi[i] = sp;
 }
@@ -1048,9 +1133,13 @@ __global__ void k_rk_final(const double* __restrict__ y0, FinalArgs fa, const do
   const double b[5] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0, 0.0};
   const double e[5] = {1.0 / 6.0, 2.0 / 3.0, 0.0, 0.0, 1.0 / 6.0};
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double mnew[5] = {0, 0, 0, 0, 0}, merr[5] = {0, 0, 0, 0, 0};
+  // maxima of magnitudes as integers: the bits of non-negative doubles order
+  // as their values, a NaN above all of them (as nan_max keeps it)
+  unsigned long long mn = 0, me = 0;
+  int arr = 0;
   if (i < n) {
     double db = 0.0, de = 0.0;
+#pragma unroll
     for (int j = 0; j < 5; ++j) {
       const double kv = fa.k[j][i];
       db = db + kv * b[j];
@@ -1058,36 +1147,53 @@ __global__ void k_rk_final(const double* __restrict__ y0, FinalArgs fa, const do
     }
     const double yn = y0[i] + h * db;
     ynew[i] = yn;
-    int arr = 0;
     while (arr < 9 && i >= fa.off[arr + 1]) ++arr;
-    // G1, G2, a_add_1, a_add_2, a_add_3 enter the error norm
-    int slot = -1;
-    if (arr == S_G1) slot = 0;
-    else if (arr == S_G2) slot = 1;
-    else if (arr == S_AADD1) slot = 2;
-    else if (arr == S_AADD2) slot = 3;
-    else if (arr == S_AADD3) slot = 4;
-    if (slot >= 0) {
-      mnew[slot] = fabs(yn);
-      merr[slot] = fabs((de - db) * h);
-    }
+    mn = abs_bits(yn);
+    me = abs_bits((de - db) * h);
   }
+  // G1, G2, a_add_1, a_add_2, a_add_3 enter the error norm.  A block meets one
+  // or two arrays: only their maxima are reduced.
+  __shared__ unsigned long long sh[2][32];
+  const long long i0 = blockIdx.x * (long long)blockDim.x, i1 = min(i0 + (long long)blockDim.x, n);
   for (int s = 0; s < 5; ++s) {
-    const double m1 = block_reduce<1>(mnew[s]);
-    if (threadIdx.x == 0) part[blockIdx.x * 10 + s] = m1;
-    const double m2 = block_reduce<1>(merr[s]);
-    if (threadIdx.x == 0) part[blockIdx.x * 10 + 5 + s] = m2;
+    const int a = s == 0 ? S_G1 : (s == 1 ? S_G2 : (s == 2 ? S_AADD1 : (s == 3 ? S_AADD2 : S_AADD3)));
+    unsigned long long vn = 0, ve = 0;
+    if (fa.off[a] < i1 && fa.off[a + 1] > i0) {
+      if (i < n && arr == a) {
+        vn = mn;
+        ve = me;
+      }
+      block_max2(vn, ve, sh);
+    }
+    if (threadIdx.x == 0) {
+      part[blockIdx.x * 10 + s] = __longlong_as_double((long long)vn);
+      part[blockIdx.x * 10 + 5 + s] = __longlong_as_double((long long)ve);
+    }
   }
 }
 
-__global__ void k_rk_err(const double* __restrict__ part, int nblocks, double* sc) {
+__global__ void __launch_bounds__(1024) k_rk_err(const double* __restrict__ part, int nblocks, double* sc) {
   pdl_wait();
-  // one block of 32 threads: max over blocks per slot, then the norm
+  // max over blocks per slot (one warp took 719 us over the 3348 blocks of a
+  // 513 x 257 tank: its ten lanes waited for every block in turn), then the norm
+  __shared__ unsigned long long sh[10][32];
   __shared__ double mx[10];
-  if (threadIdx.x < 10) {
-    double m = 0.0;
-    for (int b = 0; b < nblocks; ++b) m = nan_max(m, part[b * 10 + threadIdx.x]);
-    mx[threadIdx.x] = m;
+  unsigned long long m[10];
+#pragma unroll
+  for (int s = 0; s < 10; ++s) m[s] = 0;
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+#pragma unroll
+    for (int s = 0; s < 10; ++s) m[s] = max(m[s], abs_bits(__ldcg(part + b * 10 + s)));
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int s = 0; s < 10; ++s) {
+    m[s] = warp_max(m[s]);
+    if (lane == 0) sh[s][w] = m[s];
+  }
+  __syncthreads();
+  if (w < 10) {
+    const unsigned long long v = warp_max(lane < nw ? sh[w][lane] : 0ULL);
+    if (lane == 0) mx[w] = __longlong_as_double((long long)v);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1130,11 +1236,12 @@ __global__ void k_rk_out(const double* __restrict__ G1, const double* __restrict
   }
   const double bs = block_reduce<0>(e);
   if (threadIdx.x == 0) part[blockIdx.x] = bs;
-  if (last_block(counter) && threadIdx.x == 0) {
-    double S = 0.0;
-    for (unsigned int b = 0; b < gridDim.x; ++b) S += __ldcg(part + b);
-    volume_fix(etam, S, sc, igeom, d_hinge, xlen);
-    *counter = 0;
+  if (last_block(counter)) {
+    const double S = sum_parts(part, (int)gridDim.x);
+    if (threadIdx.x == 0) {
+      volume_fix(etam, S, sc, igeom, d_hinge, xlen);
+      *counter = 0;
+    }
   }
 }
 
@@ -1298,10 +1405,14 @@ struct Enq {
     if (!dealias_on(order)) return;
     dealias_many({{dclass(order), buf}});
   }
+  // elementwise kernels: small blocks where 256-thread ones would leave SMs
+  // idle (a warp's FP64 operation takes 64 cycles of its scheduler: the 13 blocks
+  // of a 2-D tank's 3075 points did k_group_products in 5.2 us, k_assemble in 4.4)
   template <typename K, typename... A>
   void ew(K kern, long long n, A... a) {
     if (n <= 0) return;
-    launch_pdl(kern, dim3(nblk(n)), dim3(kEW), 0, st, a...);
+    const int t = n <= 148LL * kEW ? kTrig : kEW;
+    launch_pdl(kern, dim3(nblk(n, t)), dim3(t), 0, st, a...);
   }
   template <typename K, typename... A>
   void ew_trig(K kern, long long n, A... a) {
@@ -1392,9 +1503,11 @@ void enqueue_sweet2(Ctx& c, Enq& W, const double* y, double* k) {
   for (int q = 0; q < 6; ++q) wo.w[q] = n2 == 1 ? w[W2_WF + q] : w[W2_WFM + q];
   launch_pdl(k_wmk_from_fs, dim3(n3, n2), dim3(128), 0, sw, a1, da1, (const double*)d.kx2cshx,
              (const double*)d.kycshx, (const double*)d.kshx, n1, n2, n3, wo);
-  if (n2 != 1)
-    for (int q = 0; q < 6; ++q)
-      launch_y_f2s(W.tb, w[W2_WFM + q], n3, n3, w[W2_WF + q], n3, (q == 2 || q == 3) ? 1 : 0, sw);
+  if (n2 != 1) {
+    std::vector<YReq> ys;
+    for (int q = 0; q < 6; ++q) ys.push_back(YReq{w[W2_WFM + q], w[W2_WF + q], (q == 2 || q == 3) ? 1 : 0});
+    launch_y_f2s(W.tb, ys, n3, n3, n3, sw);
+  }
   D1stArgs g{};
   for (int q = 0; q < 9; ++q) g.T[q] = w[W2_T9 + q];
   for (int f = 0; f < W_NF; ++f) g.F[f] = w[W2_F + f];
@@ -1432,8 +1545,7 @@ void enqueue_sweet2(Ctx& c, Enq& W, const double* y, double* k) {
              (const double*)d.kxcsh, n1, n2, n3a, n2 == 1 ? w[W2_P2T] : w[W2_P2TM],
              n2 == 1 ? w[W2_P2Z] : w[W2_P2ZM]);
   if (n2 != 1) {
-    launch_y_f2s(W.tb, w[W2_P2TM], n1, n1, w[W2_P2T], n1, 0, sw);
-    launch_y_f2s(W.tb, w[W2_P2ZM], n1, n1, w[W2_P2Z], n1, 0, sw);
+    launch_y_f2s(W.tb, {YReq{w[W2_P2TM], w[W2_P2T], 0}, YReq{w[W2_P2ZM], w[W2_P2Z], 0}}, n1, n1, n1, sw);
   }
   // phidphiz of the second order and the free-surface conditions
   W.ew(k_mul, nN, y + L.off[S_A2ND], (const double*)d.kth1, 1.0, w[W2_A2K], nN);
@@ -1483,9 +1595,11 @@ void enqueue_sweet3(Ctx& c, Enq& W, const double* y, double* k) {
   for (int q = 0; q < 6; ++q) wo.w[q] = n2 == 1 ? w[W2_WF2 + q] : w[W2_WFM2 + q];
   launch_pdl(k_wmk_from_fs, dim3(n3, n2), dim3(128), 0, sw, y + L.off[S_A2ND], (const double*)(k + L.off[S_A2ND]),
              (const double*)d.kx2cshx, (const double*)d.kycshx, (const double*)d.kshx, n1, n2, n3, wo);
-  if (n2 != 1)
-    for (int q = 0; q < 6; ++q)
-      launch_y_f2s(W.tb, w[W2_WFM2 + q], n3, n3, w[W2_WF2 + q], n3, (q == 2 || q == 3) ? 1 : 0, sw);
+  if (n2 != 1) {
+    std::vector<YReq> ys;
+    for (int q = 0; q < 6; ++q) ys.push_back(YReq{w[W2_WFM2 + q], w[W2_WF2 + q], (q == 2 || q == 3) ? 1 : 0});
+    launch_y_f2s(W.tb, ys, n3, n3, n3, sw);
+  }
   Sweet3Wmk sv{};
   for (int q = 0; q < 6; ++q) {
     sv.x1[q] = w[W2_WA3 + q];
@@ -1563,10 +1677,12 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
                  (const double*)kA1, (const double*)d.cosk, (const double*)d.sink, (const double*)d.kx_add,
                  (const double*)d.k_add, (const double*)d.ky, (const double*)d.csh, (const double*)d.ksh,
                  (const double*)d.kycsh, (const double*)d.kxcsh, n1, n2, P.n3a, co);
-      if (n2 != 1)
+      if (n2 != 1) {
+        std::vector<YReq> ys;
         for (int f = 0; f < W_NF; ++f)
-          launch_y_f2s(W.tb, d.w2[W2_FM + f], n1, n1, d.w2[W2_F + f], n1,
-                       (f == W_Y || f == W_YT || f == W_YZ) ? 1 : 0, sw);
+          ys.push_back(YReq{d.w2[W2_FM + f], d.w2[W2_F + f], (f == W_Y || f == W_YT || f == W_YZ) ? 1 : 0});
+        launch_y_f2s(W.tb, ys, n1, n1, n1, sw);
+      }
       phit1 = d.w2[W2_F + W_T];
       phiz1 = d.w2[W2_F + W_Z];
     } else {
@@ -1575,8 +1691,7 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
           n2 == 1 ? d.phiz_add1 : d.Q[1]);
       if (n2 != 1) {
         // y sums: sum_j2 A(i1, j2) cos(ky(j2) y(i2)) = FOURIER_2_SPACE_y
-        launch_y_f2s(W.tb, d.Q[0], n1, n1, d.phit_add1, n1, 0, sw);
-        launch_y_f2s(W.tb, d.Q[1], n1, n1, d.phiz_add1, n1, 0, sw);
+        launch_y_f2s(W.tb, {YReq{d.Q[0], d.phit_add1, 0}, YReq{d.Q[1], d.phiz_add1, 0}}, n1, n1, n1, sw);
       }
     }
     // phidphiz + SWEET_1 RHS
@@ -1634,15 +1749,21 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
            (const double*)d.ksh, (const double*)d.kycsh, (const double*)d.kxcsh, n1, n2, P.n3a,
            d.Q[0], d.Q[1], d.Q[2], d.Q[3], d.Q[4]);
       const int lines = n1 * P.n3a;
-      launch_y_f2s(W.tb, d.Q[0], lines, lines, d.B[0], lines, 0, sw);
-      launch_y_f2s(W.tb, d.Q[1], lines, lines, d.B[1], lines, 0, sw);
-      launch_y_f2s(W.tb, d.Q[2], lines, lines, d.B[2], lines, 1, sw);
-      launch_y_f2s(W.tb, d.Q[3], lines, lines, d.B[3], lines, 0, sw);
-      launch_y_f2s(W.tb, d.Q[4], lines, lines, d.B[4], lines, 0, sw);
-      W.ew(k_phiadd_contract, nN, (const double*)d.eta_sp, (const double*)d.kx_add,
-           (const double*)d.B[0], (const double*)d.B[1], (const double*)d.B[2],
-           (const double*)d.B[3], (const double*)d.B[4], n1, n2, P.n3a, d.phix_add, d.phiy_add,
-           d.phiz_add, d.phit_add, d.phi_add);
+      {
+        std::vector<YReq> ys;
+        for (int q = 0; q < 5; ++q) ys.push_back(YReq{d.Q[q], d.B[q], q == 2 ? 1 : 0});
+        launch_y_f2s(W.tb, ys, lines, lines, lines, sw);
+      }
+      // a point's modes shared by eight threads below 150 k points: 8192 points
+      // 66 us in one thread each with a sincos per mode
+      auto contract = [&](auto kern, int cx) {
+        launch_pdl(kern, dim3((unsigned)((nN + cx - 1) / cx)), dim3(128), 0, sw, (const double*)d.eta_sp,
+                   (const double*)d.kx_add, (const double*)d.B[0], (const double*)d.B[1], (const double*)d.B[2],
+                   (const double*)d.B[3], (const double*)d.B[4], n1, n2, P.n3a, d.phix_add, d.phiy_add, d.phiz_add,
+                   d.phit_add, d.phi_add);
+      };
+      if (nN < 32768) contract(k_phiadd_contract<8>, 16);
+      else contract(k_phiadd_contract<1>, 128);
     }
   }
   // without a wavemaker phi_add and its derivatives stay zero (zero-filled
@@ -1667,7 +1788,10 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
       int jend = j + 1;
       while (jend < M && !E.dealias_on(jend)) ++jend;
       PowArgs pa{};
-      for (int t = 0; t < M; ++t) pa.e[t] = d.etapm[t];
+      for (int t = 0; t < M; ++t) {
+        pa.e[t] = d.etapm[t];
+        pa.inv[t] = 1.0 / (t + 1);
+      }
       pa.j0 = j;
       pa.j1 = jend;
       Pw.ew(k_pow_run, nB, pa, nB);
@@ -1825,6 +1949,22 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
     gt.nterm++;
   }
   gt.ngroup = (int)gkind.size();
+  {
+    // sort by group, keeping the order inside each group
+    GroupTerms u = gt;
+    int n = 0;
+    for (int g = 0; g < gt.ngroup; ++g) {
+      gt.start[g] = n;
+      for (int t = 0; t < u.nterm; ++t)
+        if (u.group[t] == g) {
+          gt.x[n] = u.x[t];
+          gt.y[n] = u.y[t];
+          gt.s[n] = u.s[t];
+          gt.group[n++] = g;
+        }
+    }
+    gt.start[gt.ngroup] = n;
+  }
   for (int g = 0; g < gt.ngroup; ++g) gt.out[g] = d.grp[g];
   AssembleArgs aa{};
   aa.ng1 = aa.ng2 = aa.nt1 = 0;
@@ -1955,7 +2095,7 @@ void enqueue_step(Ctx& c, cudaStream_t st) {
   fa.off[10] = S;
   const int nb = nblk(S);
   launch_pdl(k_rk_final, dim3(nb), dim3(kEW), 0, st, d.y0, fa, d.sc, d.ynew, d.part, S);
-  launch_pdl(k_rk_err, dim3(1), dim3(32), 0, st, d.part, nb, d.sc);
+  launch_pdl(k_rk_err, dim3(1), dim3(nb > 256 ? 1024 : 320), 0, st, d.part, nb, d.sc);
   launch_pdl(k_rk_out, dim3(nblk(nN, kTrig)), dim3(kTrig), 0, st, d.ynew + L.off[S_G1], d.ynew + L.off[S_G2],
                                      d.k[4] + L.off[S_G1], d.k[4] + L.off[S_G2], d.omega, d.sc,
                                      (int)nN, P.igeom, P.d_hinge, P.xlen, d.etam, d.phim, d.NL1,

@@ -511,6 +511,76 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
   }
 }
 
+// y pass of few lines (the wavemaker grids of narrow 3-D tanks): CTA = (job, 32
+// lines, two lane outputs), lane = line, the 8 warps split the inputs, so that a
+// warp's inputs have one parity and the sums E, O of mode 1 are sums over warps.
+// One thread per line with eight outputs left this to two CTAs of one warp: 20 us
+// for 30 lines of 32 points, 3.4 us here.
+constexpr int kFewLines = 32;
+template <int NJ>
+__global__ void __launch_bounds__(256) axis_pass_few_lines(const AxisBatchT<NJ> b) {
+  __shared__ double red[2][8][32];
+  int jb = 0;
+  while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
+  const AxisJob& J = b.job[jb];
+  const int D = J.D, D4 = 4 * D;
+  const bool paired = J.mode == 1;
+  const int ngrp = (J.nlane + 1) / 2;
+  const int local = blockIdx.x - b.start[jb];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k0 = 2 * (local % ngrp), line = (local / ngrp) * 32 + lane;
+  const bool on = line < J.nlines;
+  const double* __restrict__ x = J.in + (long long)(on ? line : 0) * J.in_sl;
+  const double* __restrict__ wr = J.win ? J.win + (long long)(on ? line : 0) * J.win_sl : nullptr;
+  const int jlo = J.jlo, j_end = min(J.jhi, J.nin);
+  const bool is_sin = J.off != 0;
+  int m[2], inc[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    m[r] = mod4d(2LL * (jlo + warp) * (k0 + r) + J.off, D4);
+    inc[r] = mod4d(16LL * (k0 + r), D4);
+  }
+  pdl_wait();
+  double acc[2] = {0.0, 0.0};
+  if (on) {
+#pragma unroll 4
+    for (int j = jlo + warp; j < j_end; j += 8) {
+      double v = in_at(x, J.in_sk, wr, J.win_sk, j);
+      // end inputs count full or half of an interior one
+      if ((j == 0 && J.w0 != J.wm) || (j == J.N - 1 && J.wl != J.wm)) v *= 0.5;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        acc[r] = fma(v, twiddle(J.q, D, m[r]), acc[r]);
+        m[r] += inc[r];
+        if (m[r] >= D4) m[r] -= D4;
+      }
+    }
+  }
+  red[0][warp][lane] = acc[0];
+  red[1][warp][lane] = acc[1];
+  __syncthreads();
+  if (warp >= 2 || !on) return;
+  const int k = k0 + warp;
+  if (k >= J.nlane) return;
+  double s[2] = {0.0, 0.0};  // over the warps of even and of odd inputs
+#pragma unroll
+  for (int w = 0; w < 8; w += 2) {
+    s[0] += red[warp][w][lane];
+    s[1] += red[warp][w + 1][lane];
+  }
+  const double e = (jlo & 1) ? s[1] : s[0], o = (jlo & 1) ? s[0] : s[1];
+  auto put = [&](int kk, double v) {
+    if (kk >= J.nout) return;
+    const double sc = ((kk == 0) ? J.s0 : ((kk == J.N - 1) ? J.sl : J.sm)) * J.gscale * J.wm;
+    const double y = (kk >= J.klo && kk < J.khi) ? v * sc : 0.0;
+    const long long at = (long long)line * J.out_sl + (long long)kk * J.out_sk;
+    J.out[at] = y;
+    if (J.epi) acc_epilogue(b.acc, at, y);
+  };
+  put(k, e + o);
+  if (paired && D - k != k) put(D - k, is_sin ? o - e : e - o);
+}
+
 // Two-level passes for REDFT00 / RODFT00 kinds when D = A * B.  With
 // j = B j1 + j2, pi j k / D = pi j1 k / A + pi j2 k / D, so
 //   cos-kind: y_k = sum_j2 [cos(pi j2 k/D) C(j2,k) - sin(pi j2 k/D) S(j2,k)]
@@ -1777,6 +1847,34 @@ void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
   }
   if (bf.njobs) launch_fft_jobs(bf, fplan, tb, st);
   if (b2.njobs) launch_ytl(b2, tb.q_const, st);
+  {
+    // few lines
+    AxisBatch few{}, rest{};
+    few.njobs = rest.njobs = 0;
+    few.acc = rest.acc = b.acc;
+    int total = 0;
+    for (int i = 0; i < b.njobs; ++i) {
+      AxisJob J = b.job[i];
+      const bool c1s1 = (J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0);
+      if (!c1s1 || J.nlines > kFewLines || J.D < 4) {
+        rest.job[rest.njobs++] = J;
+        continue;
+      }
+      J.mode = J.nout == J.N ? 1 : 0;
+      J.nlane = J.mode ? J.D / 2 + 1 : J.nout;
+      g_xform_fmas += (double)J.nlines * J.nlane * (std::min(J.jhi, J.nin) - J.jlo);
+      few.start[few.njobs] = total;
+      total += (J.nlines + 31) / 32 * ((J.nlane + 1) / 2);
+      few.job[few.njobs++] = J;
+    }
+    few.start[few.njobs] = total;
+    if (total > 0)
+      with_capacity(few.njobs, [&](auto c) {
+        constexpr int NJ = decltype(c)::value;
+        launch_pdl(axis_pass_few_lines<NJ>, dim3(total), dim3(256), 0, st, shrink<NJ>(few));
+      });
+    b = rest;
+  }
   if (b.njobs == 0) return;
   int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
@@ -2020,25 +2118,30 @@ double measure_fp64_peak_gflops() {
   return flops / (best * 1e-3) / 1e9;
 }
 
-void launch_y_f2s(const Tables& tb, const double* in, int nlines, long long y_stride, double* out,
-                  long long out_y_stride, int cs, cudaStream_t st) {
-  AxisBatch b{};
-  b.njobs = 1;
-  AxisJob& J = b.job[0];
-  set_kind(J, cs ? K_S1_F2S : K_C1_F2S, tb.n2, tb.q_n2);
-  J.ty = tb.ty_n2[cs ? 1 : 0];
-  J.ldy = tb.ldy_n2;
-  J.in = in;
-  J.in_sk = y_stride;
-  J.in_sl = 1;
-  J.nin = tb.n2;
-  J.nlines = nlines;
-  J.nout = tb.n2;
-  J.out = out;
-  J.out_sk = out_y_stride;
-  J.out_sl = 1;
-  J.gscale = 1.0;
-  launch_batch_y(b, tb, st);
+void launch_y_f2s(const Tables& tb, const std::vector<YReq>& reqs, int nlines, long long y_stride,
+                  long long out_y_stride, cudaStream_t st) {
+  for (size_t r0 = 0; r0 < reqs.size(); r0 += kMaxJobs) {
+    AxisBatch b{};
+    b.njobs = (int)std::min<size_t>(kMaxJobs, reqs.size() - r0);
+    for (int i = 0; i < b.njobs; ++i) {
+      const YReq& r = reqs[r0 + i];
+      AxisJob& J = b.job[i];
+      set_kind(J, r.cs ? K_S1_F2S : K_C1_F2S, tb.n2, tb.q_n2);
+      J.ty = tb.ty_n2[r.cs ? 1 : 0];
+      J.ldy = tb.ldy_n2;
+      J.in = r.in;
+      J.in_sk = y_stride;
+      J.in_sl = 1;
+      J.nin = tb.n2;
+      J.nlines = nlines;
+      J.nout = tb.n2;
+      J.out = r.out;
+      J.out_sk = out_y_stride;
+      J.out_sl = 1;
+      J.gscale = 1.0;
+    }
+    launch_batch_y(b, tb, st);
+  }
 }
 
 }  // namespace hos
