@@ -227,6 +227,12 @@ void launch_transforms(const XfReq* reqs, int nreq, const Tables& tb, double* co
                        cudaStream_t st);
 
 struct Tables;
+// The transform of nlines contiguous lines of n points with tb's table q_n1 and
+// scratch part (transform_noalloc).
+void launch_lines(const Tables& tb, int dir, int cs, int n, int nlines, const double* in, double* out,
+                  cudaStream_t st);
+// Whether launch_lines runs them without split sums (direct_pass).
+bool lines_direct(int n, int nlines);
 // F2S along y only (FOURIER_2_SPACE_y, fourier_FFTW.f90:340-428) of fields of
 // nlines lines that are contiguous in memory, all in one launch; cs: 0 cos, 1 sin.
 struct YReq {

@@ -89,9 +89,12 @@ extern "C" int hosnwt_transform_noalloc(int dir, int cs, int n, int nlines, cons
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return HOSNWT_ERR_CUDA;
-  // the counters must start at zero; the table is rebuilt for this length
-  if (cudaMemsetAsync(cnt, 0, sizeof(unsigned int) * kCntLen, st) != cudaSuccess) return HOSNWT_ERR_CUDA;
-  k_noalloc_table<<<(n + 255) / 256, 256, 0, st>>>(q, n - 1);
+  // the counters of split sums must start at zero (sums of up to 513 terms, and
+  // those of few lines, are not split); the table is rebuilt for this length, in
+  // small blocks: a cospi is some forty FP64 operations of 64 cycles a warp
+  const bool may_split = n > 513 && !lines_direct(n, nlines);
+  if (may_split && cudaMemsetAsync(cnt, 0, sizeof(unsigned int) * kCntLen, st) != cudaSuccess) return HOSNWT_ERR_CUDA;
+  k_noalloc_table<<<(n + 31) / 32, 32, 0, st>>>(q, n - 1);
   if (cudaGetLastError() != cudaSuccess) return HOSNWT_ERR_CUDA;
   Tables tb{};
   tb.n1 = n;
@@ -106,27 +109,6 @@ extern "C" int hosnwt_transform_noalloc(int dir, int cs, int n, int nlines, cons
   tb.cnt = cnt;
   tb.cnt_cap = kCntLen;
   tb.q_const = false;  // the table kernel above runs right before the passes
-  double* no_tmp[kMaxJobs] = {};
-  XfReq rq[kMaxJobs];
-  for (int l0 = 0; l0 < nlines; l0 += kMaxJobs) {
-    const int cntl = (nlines - l0 < kMaxJobs) ? nlines - l0 : kMaxJobs;
-    for (int i = 0; i < cntl; ++i) {
-      XfReq& r = rq[i];
-      r.grid = GRID_N;
-      r.dir = dir;
-      r.csx = cs;
-      r.csy = 0;
-      r.in = in + (long long)(l0 + i) * n;
-      r.in_ld = n;
-      r.nin1 = n;
-      r.nin2 = 1;
-      r.out = out + (long long)(l0 + i) * n;
-      r.out_ld = n;
-      r.nout1 = n;
-      r.nout2 = 1;
-      r.scale = 1.0;
-    }
-    launch_transforms(rq, cntl, tb, no_tmp, st);
-  }
+  launch_lines(tb, dir, cs, n, nlines, in, out, st);
   return cudaGetLastError() == cudaSuccess ? HOSNWT_OK : HOSNWT_ERR_CUDA;
 }

@@ -581,6 +581,121 @@ __global__ void __launch_bounds__(256) axis_pass_few_lines(const AxisBatchT<NJ> 
   if (paired && D - k != k) put(D - k, is_sin ? o - e : e - o);
 }
 
+// scale of output k; w: the interior weight, where pass 1 left it out
+__device__ __forceinline__ double p2_scale(const AxisJob& J, int k, double w) {
+  return ((k == 0) ? J.s0 : ((k == J.N - 1) ? J.sl : J.sm)) * J.gscale * w;
+}
+__device__ __forceinline__ void p2_put(const AxisJob& J, const AccEpi& acc, int line, int k, double y, double scale) {
+  if (k >= J.nout) return;
+  const bool on = k >= J.klo && k < J.khi;
+  const long long e = (long long)line * J.out_sl + (long long)k * J.out_sk;
+  const double v = on ? y * scale : 0.0;
+  J.out[e] = v;
+  if (J.epi) acc_epilogue(acc, e, v);
+}
+
+// x or -x by the sign bit
+__device__ __forceinline__ double flip_if(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// Direct x pass of few lines (lengths that do not factor, 2-D tanks): CTA = (job,
+// line, KO lane outputs); a warp holds KO outputs times 32 / KO slices of the sum,
+// warp w the slices w, w + 4, ..., which meet by shuffles and in shared memory.  The
+// quarter-wave table is staged before the wait for the previous kernel, and no
+// FP64 operation but the FMAs of the sums is in the loop: a warp's holds its
+// scheduler for 64 cycles, under which the index arithmetic of the next twiddle
+// is free (a staged tile of the CTA's twiddles cost 40 instructions each, and an
+// ensemble of six tanks 15 %).  With mode 1 a slice's inputs have one parity (an even
+// number of slices): the sums E, O of the k <-> D - k pairs; with mode 2 (every
+// input, truncated outputs) the slices run over u = x_j + x_{D-j} or v = x_j -
+// x_{D-j}.  D = 257, one line: 5.8 us by axis_pass_lanes_k (9 CTAs), 3.6 us here.
+constexpr int kDirThreads = 128;
+constexpr int kDirMaxD = 4200;      // table and inputs within 100 KB
+constexpr int kDirMaxLines = 8;     // more lines fill the SMs by axis_pass_lanes_k
+__host__ __device__ inline int dir_terms(const AxisJob& J) {  // lane terms of the sum
+  return J.mode == 2 ? J.D / 2 + 1 : (J.jhi < J.nin ? J.jhi : J.nin);
+}
+template <int NJ, int KO>
+__global__ void __launch_bounds__(kDirThreads) direct_pass(const AxisBatchT<NJ> b) {
+  extern __shared__ double smd[];
+  __shared__ double red[4][KO];
+  constexpr int SL = 4 * (32 / KO);
+  int jb = 0;
+  while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
+  const AxisJob& J = b.job[jb];
+  const int D = J.D, D4 = 4 * D, mode = J.mode;
+  const int nkb = (J.nlane + KO - 1) / KO;
+  const int local = blockIdx.x - b.start[jb];
+  const int line = local / nkb, k0 = (local - line * nkb) * KO;
+  const int jlo = J.jlo, j_end = min(J.jhi, J.nin), nt = dir_terms(J);
+  const bool is_sin = J.off != 0;
+  double* tq = smd;             // cos(pi m / (2 D)), m = 0 .. D
+  double* xs = smd + D + 1;     // inputs, or u then v
+  const double* __restrict__ q = J.q;
+  auto stage_twiddles = [&]() {
+    for (int t = threadIdx.x; t <= D; t += kDirThreads) tq[t] = __ldg(q + t);
+  };
+  if (b.early) stage_twiddles();
+  const double* __restrict__ x = J.in + (long long)line * J.in_sl;
+  const double* __restrict__ wr = J.win ? J.win + (long long)line * J.win_sl : nullptr;
+  const bool half0 = J.w0 != J.wm, halfD = J.wl != J.wm;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kl = lane % KO, slice = warp + 4 * (lane / KO);
+  const int k = k0 + kl;
+  const double sk = p2_scale(J, k, J.wm), sm = p2_scale(J, D - k, J.wm);
+  const long long in_sk = J.in_sk, win_sk = J.win_sk;
+  pdl_wait();
+  if (!b.early) stage_twiddles();
+  auto u = [&](int j) -> double {
+    if (j < jlo || j >= j_end) return 0.0;
+    double v = in_at(x, in_sk, wr, win_sk, j);
+    if ((j == 0 && half0) || (j == D && halfD)) v *= 0.5;
+    return v;
+  };
+  for (int j = threadIdx.x; j < nt; j += kDirThreads) {
+    const double v = u(j);
+    if (mode == 2) {
+      const bool mid = 2 * j == D;
+      const double m = mid ? 0.0 : u(D - j);
+      xs[j] = v + m;
+      xs[nt + j] = v - m;
+    } else {
+      xs[j] = v;
+    }
+  }
+  __syncthreads();
+  // cos: even k sees u, odd k sees v; sin the other way round
+  const double* xp = xs + (mode == 2 && (((k & 1) == 0) == is_sin) ? nt : 0);
+  int m = mod4d(2LL * slice * k + J.off, D4);
+  const int inc = mod4d(2LL * SL * k, D4);
+  auto next = [&]() -> double {
+    const int mm = m > 2 * D ? D4 - m : m;
+    const bool neg = mm > D;
+    m += inc;
+    if (m >= D4) m -= D4;
+    return flip_if(tq[neg ? 2 * D - mm : mm], neg);
+  };
+  double acc = 0.0, acc2 = 0.0;  // two chains
+  int j = slice;
+#pragma unroll 2
+  for (; j + SL < nt; j += 2 * SL) {
+    acc = fma(xp[j], next(), acc);
+    acc2 = fma(xp[j + SL], next(), acc2);
+  }
+  if (j < nt) acc = fma(xp[j], next(), acc);
+  acc += acc2;
+#pragma unroll
+  for (int off = KO; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (lane < KO) red[warp][lane] = acc;
+  __syncthreads();
+  if (threadIdx.x < KO && k < J.nlane) {
+    const double e = red[0][lane] + red[2][lane], o = red[1][lane] + red[3][lane];
+    p2_put(J, b.acc, line, k, e + o, sk);
+    if (mode == 1 && D - k != k) p2_put(J, b.acc, line, D - k, is_sin ? o - e : e - o, sm);
+  }
+}
+
 // Two-level passes for REDFT00 / RODFT00 kinds when D = A * B.  With
 // j = B j1 + j2, pi j k / D = pi j1 k / A + pi j2 k / D, so
 //   cos-kind: y_k = sum_j2 [cos(pi j2 k/D) C(j2,k) - sin(pi j2 k/D) S(j2,k)]
@@ -628,11 +743,6 @@ __host__ __device__ inline P1Shape p1_shape(int A, int B, int K, int P) {
   s.kblocks = (p1_half(A) + s.nk) / s.nk;
   s.jblocks = (B + s.G - 1) / s.G;
   return s;
-}
-
-// x or -x by the sign bit
-__device__ __forceinline__ double flip_if(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
 }
 
 // pass 1: CTA = (job, line, nk values of k', G values of j2).  The even and odd
@@ -740,19 +850,6 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
 // y(k).  Lanes own k <= D/2, and the sums E, O over even and odd j2 give y(k)
 // = E + O and y(D - k) = E - O (cos kind) or O - E (sin kind).
 __host__ __device__ inline int p2_lanes(const AxisJob& J) { return J.mode == 1 ? J.D / 2 + 1 : J.nout; }
-
-// scale of output k; w: the interior weight, where pass 1 left it out
-__device__ __forceinline__ double p2_scale(const AxisJob& J, int k, double w) {
-  return ((k == 0) ? J.s0 : ((k == J.N - 1) ? J.sl : J.sm)) * J.gscale * w;
-}
-__device__ __forceinline__ void p2_put(const AxisJob& J, const AccEpi& acc, int line, int k, double y, double scale) {
-  if (k >= J.nout) return;
-  const bool on = k >= J.klo && k < J.khi;
-  const long long e = (long long)line * J.out_sl + (long long)k * J.out_sk;
-  const double v = on ? y * scale : 0.0;
-  J.out[e] = v;
-  if (J.epi) acc_epilogue(acc, e, v);
-}
 
 // pass 2: CTA = (job, line, KO outputs).  A warp holds KO outputs times 32 / KO
 // slices of the j2 sum, warp w the slices w, w + 4, ...: every slice of a warp
@@ -1604,7 +1701,64 @@ bool launch_two_level_fused(AxisBatch& b, int nsm, bool early, cudaStream_t st) 
 }
 
 // Decide the symmetry mode and the split of every x-pass job, then launch.
+// Jobs of few lines whose twiddles fit run direct_pass and leave the batch.
+void launch_direct(AxisBatch& b, const Tables& tb, cudaStream_t st) {
+  AxisBatch few{}, rest{};
+  few.njobs = rest.njobs = 0;
+  few.acc = rest.acc = b.acc;
+  few.early = tb.q_const ? 1 : 0;
+  long long lanes = 0;
+  for (int i = 0; i < b.njobs; ++i) {
+    AxisJob J = b.job[i];
+    const bool c1s1 = (J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0);
+    J.mode = J.nout == J.N ? 1 : (J.nin >= J.N ? 2 : 0);
+    J.nlane = J.mode == 1 ? J.D / 2 + 1 : J.nout;
+    if (!c1s1 || J.D < 4 || J.nlines > kDirMaxLines || J.D > kDirMaxD) {
+      rest.job[rest.njobs++] = b.job[i];
+      continue;
+    }
+    lanes += (long long)J.nlines * J.nlane;
+    few.job[few.njobs++] = J;
+  }
+  b = rest;
+  if (few.njobs == 0) return;
+  // fewer outputs per CTA until the launch covers the SMs
+  int KO = 32;
+  while (KO > 4 && lanes / KO < std::max(tb.nsm, 1)) KO /= 2;
+  int total = 0;
+  size_t smem = 0;
+  for (int i = 0; i < few.njobs; ++i) {
+    const AxisJob& J = few.job[i];
+    const int nt = dir_terms(J);
+    few.start[i] = total;
+    total += J.nlines * ((J.nlane + KO - 1) / KO);
+    smem = std::max(smem, sizeof(double) * ((size_t)J.D + 1 + (J.mode == 2 ? 2 : 1) * (size_t)nt));
+    g_xform_fmas += (double)J.nlines * J.nlane * nt;
+  }
+  few.start[few.njobs] = total;
+  static PerDeviceOnce attr;
+  attr.run([&] {
+    for (int nj : {1, 2, 4, 8, kMaxJobs})
+      with_capacity(nj, [&](auto c) {
+        constexpr int NJ = decltype(c)::value;
+        allow_smem(direct_pass<NJ, 4>);
+        allow_smem(direct_pass<NJ, 8>);
+        allow_smem(direct_pass<NJ, 16>);
+        allow_smem(direct_pass<NJ, 32>);
+      });
+  });
+  with_capacity(few.njobs, [&](auto c) {
+    constexpr int NJ = decltype(c)::value;
+    if (KO == 4) launch_pdl(direct_pass<NJ, 4>, dim3(total), dim3(kDirThreads), smem, st, shrink<NJ>(few));
+    else if (KO == 8) launch_pdl(direct_pass<NJ, 8>, dim3(total), dim3(kDirThreads), smem, st, shrink<NJ>(few));
+    else if (KO == 16) launch_pdl(direct_pass<NJ, 16>, dim3(total), dim3(kDirThreads), smem, st, shrink<NJ>(few));
+    else launch_pdl(direct_pass<NJ, 32>, dim3(total), dim3(kDirThreads), smem, st, shrink<NJ>(few));
+  });
+}
+
 void launch_batch_x(AxisBatch& b, const Tables& tb, cudaStream_t st) {
+  launch_direct(b, tb, st);
+  if (b.njobs == 0) return;
   b.early = tb.q_const ? 1 : 0;
   long long tiles_total = 0;
   for (int i = 0; i < b.njobs; ++i) {
@@ -2116,6 +2270,44 @@ double measure_fp64_peak_gflops() {
   cudaFree(out);
   const double flops = 2.0 * 8.0 * iters * (double)blocks * threads;
   return flops / (best * 1e-3) / 1e9;
+}
+
+bool lines_direct(int n, int nlines) { return nlines <= kDirMaxLines && n - 1 <= kDirMaxD; }
+
+// nlines contiguous lines of n points (no context): two-level passes in chunks
+// that fit the scratch tb.part where the length factors, else the direct sums.
+void launch_lines(const Tables& tb, int dir, int cs, int n, int nlines, const double* in, double* out,
+                  cudaStream_t st) {
+  AxisJob J{};
+  set_kind(J, axis_kind(0, dir, cs), n, tb.q_n1);
+  J.nin = J.nout = n;
+  J.in_sk = J.out_sk = 1;
+  J.in_sl = J.out_sl = n;
+  J.gscale = 1.0;
+  int A = 0, B = 0;
+  if (nlines >= 4) pick_factors(J.D, n, n, &A, &B);
+  const long long per = (long long)B * (A + 1) * 2;
+  const long long chunk = A > 0 ? tb.part_cap / per : 0;
+  const bool two = chunk >= std::min(nlines, 16);
+  const int step = two ? (int)std::min<long long>(chunk, nlines) : nlines;
+  for (int l0 = 0; l0 < nlines; l0 += step) {
+    AxisBatch b{};
+    b.njobs = 1;
+    b.job[0] = J;
+    AxisJob& X = b.job[0];
+    X.in = in + (long long)l0 * n;
+    X.out = out + (long long)l0 * n;
+    X.nlines = std::min(step, nlines - l0);
+    if (two) {
+      X.A = A;
+      X.B = B;
+      X.mode = (B % 2 == 0) ? 1 : 0;
+      X.cs = tb.part;
+      launch_two_level(b, tb.nsm, tb.q_const, st);
+    } else {
+      launch_batch_x(b, tb, st);
+    }
+  }
 }
 
 void launch_y_f2s(const Tables& tb, const std::vector<YReq>& reqs, int nlines, long long y_stride,
