@@ -730,14 +730,10 @@ __host__ __device__ inline int p1_half(int A) { return A / 2; }
 struct P1Shape {
   int nk, G, kblocks, jblocks;
 };
-__host__ __device__ inline P1Shape p1_shape(int A, int B, int K, int P) {
+__host__ __device__ inline P1Shape p1_shape(int A, int B, int P) {
   P1Shape s;
   const int items = kP1Threads / P;
-  // the twiddles of nk values within 96 KB
-  int cap = 96 * 1024 / (16 * (K + 1));
-  if (cap < 1) cap = 1;
   s.nk = p1_half(A) + 1 < items ? p1_half(A) + 1 : items;
-  if (s.nk > cap) s.nk = cap;
   s.G = items / s.nk;
   if (s.G > B) s.G = B;
   s.kblocks = (p1_half(A) + s.nk) / s.nk;
@@ -749,7 +745,7 @@ __host__ __device__ inline P1Shape p1_shape(int A, int B, int K, int P) {
 // j1 terms are summed apart: cos / sin(pi j1 (A - k') / A) = +-(-1)^j1 cos /
 // sin(pi j1 k' / A), so the same four sums give C, S at k' and at A - k' and
 // half of the k' are computed.  Threads own (k', j2, part) with k' fastest:
-// twiddles are read without bank conflicts, inputs are broadcast.  The inputs
+// inputs are broadcast, twiddles gathered from the 2 A pairs cos, sin(pi m / A).  The inputs
 // enter with the interior weight 1; pass 2 multiplies the outputs by it.
 template <int NJ>
 __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<NJ> b, int P) {
@@ -758,26 +754,23 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
   int jb = 0;
   while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
   const AxisJob& J = b.job[jb];
-  const int A = J.A, B = J.B, D = J.D, D4 = 4 * D, H = p1_half(A);
+  const int A = J.A, B = J.B, D = J.D, H = p1_half(A);
   const int j_end = min(J.jhi, J.nin), jlo = J.jlo;  // terms j in [jlo, j_end)
   const int K = (j_end + B - 1) / B, Kp = (K + 1) & ~1;
-  const P1Shape sh = p1_shape(A, B, K, P);
+  const P1Shape sh = p1_shape(A, B, P);
   int local = blockIdx.x - b.start[jb];
   const int kb = local % sh.kblocks;
   local /= sh.kblocks;
   const int j20 = (local % sh.jblocks) * sh.G, line = local / sh.jblocks;
   const int kp0 = kb * sh.nk, nk = min(sh.nk, H + 1 - kp0), G = min(sh.G, B - j20);
-  double2* tw = reinterpret_cast<double2*>(sm1);                    // [j1][k'] cos, sin(pi j1 k' / A)
-  double* xs = sm1 + 2 * (size_t)Kp * sh.nk;                        // [j1][j2] inputs, zero outside the sum
+  double2* tw = reinterpret_cast<double2*>(sm1);                    // cos, sin(pi m / A), m < 2 A
+  double* xs = sm1 + 4 * (size_t)A;                                 // [j1][j2] inputs, zero outside the sum
   const double* __restrict__ x = J.in + (long long)line * J.in_sl;
   const double* __restrict__ wr = J.win ? J.win + (long long)line * J.win_sl : nullptr;
   const double* __restrict__ q = J.q;
   auto stage_twiddles = [&]() {
-    for (int t = threadIdx.x; t < nk * Kp; t += kP1Threads) {
-      const int j1 = t / nk, kpl = t - j1 * nk;
-      // pi j1 k' / A = pi (2 B j1 k') / (2 D); both factors below 4D
-      const unsigned step = (2u * (unsigned)B * (unsigned)(kp0 + kpl)) % (unsigned)D4;
-      const int m = (int)((step * (unsigned)j1) % (unsigned)D4);
+    for (int t = threadIdx.x; t < 2 * A; t += kP1Threads) {
+      const int m = 2 * B * t;  // pi t / A = pi m / (2 D), m < 4 D
       tw[t] = make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
     }
   };
@@ -802,10 +795,16 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
   const int part = r / G, j2l = r - part * G;
   double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
   if (part < P) {
+    const int A2 = 2 * A, kp = kp0 + kpl;
+    int m = (2 * part * kp) % A2;
+    const int inc = (2 * P * kp) % A2;
 #pragma unroll 4
     for (int p = part; p < Kp / 2; p += P) {
       const double v0 = xs[2 * p * G + j2l], v1 = xs[(2 * p + 1) * G + j2l];
-      const double2 t0 = tw[2 * p * nk + kpl], t1 = tw[(2 * p + 1) * nk + kpl];
+      const int m1 = m + kp >= A2 ? m + kp - A2 : m + kp;
+      const double2 t0 = tw[m], t1 = tw[m1];
+      m += inc;
+      if (m >= A2) m -= A2;
       ce = fma(v0, t0.x, ce);
       se = fma(v0, t0.y, se);
       co = fma(v1, t1.x, co);
@@ -845,6 +844,13 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
   }
 }
 
+// cos(pi m / (2 D)) from the staged quarter-wave table, negated where neg
+__device__ __forceinline__ double twiddle_flip(const double* q, int D, int m, bool neg) {
+  const int mm = m > 2 * D ? 4 * D - m : m;
+  const bool second = mm > D;
+  return flip_if(q[second ? 2 * D - mm : mm], second != neg);
+}
+
 // Paired jobs (mode 1: B even, every output wanted): with B even, (-1)^j =
 // (-1)^j2, so y(D - k) = +-sum_j2 (-1)^j2 T_j2(k) for the terms T_j2(k) of
 // y(k).  Lanes own k <= D/2, and the sums E, O over even and odd j2 give y(k)
@@ -871,14 +877,10 @@ __global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<N
   const int line = local / nkb;
   const int k0 = (local - line * nkb) * KO;
   const double* __restrict__ q = J.q;
-  double2* tw = reinterpret_cast<double2*>(sm2);  // [j2][k] cos, sin(pi j2 k / D)
+  // the quarter-wave table: its gathers and their index arithmetic run under
+  // the FP64 operations (a staged tile of twiddles cost 70 instructions a pair)
   auto stage_twiddles = [&]() {
-    for (int t = threadIdx.x; t < B * KO; t += kP2Threads) {
-      const int j2 = t / KO, k = k0 + (t % KO);
-      // j2 < D and k < N, so 2 j2 k fits in 32 bits for N < 32768
-      const int m = (int)((2u * (unsigned)j2 * (unsigned)k) % (unsigned)D4);
-      tw[t] = make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
-    }
+    for (int t = threadIdx.x; t <= D; t += kP2Threads) sm2[t] = __ldg(q + t);
   };
   if (b.early) stage_twiddles();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -896,7 +898,10 @@ __global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<N
   // cos kind: cw C - sw S; sin kind: sw C + cw S (S with the sign of its fold)
   const bool neg = sneg != !is_sin;
   constexpr int kOwn = 8;  // terms in flight
-  double acc = 0.0;
+  double acc = 0.0, acc2 = 0.0;
+  // j2 < D and k < N, so 2 j2 k fits in 32 bits for N < 32768
+  int m = (int)((2u * (unsigned)slice * (unsigned)k) % (unsigned)D4);
+  const int inc = (int)((2u * (unsigned)SL * (unsigned)k) % (unsigned)D4);
   double2 v[kOwn];
   auto load = [&](int j2) {
 #pragma unroll
@@ -910,12 +915,18 @@ __global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<N
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) {
       if (on && j2 + i * SL < B) {
-        const double2 t = tw[(j2 + i * SL) * KO + kl];
-        acc = fma(is_sin ? t.y : t.x, v[i].x, acc);
-        acc = fma(flip_if(is_sin ? t.x : t.y, neg), v[i].y, acc);
+        // cos(pi j2 k / D) at m, sin at m - D
+        const int ms = m >= D ? m - D : m + 3 * D;
+        const double t = twiddle_flip(sm2, D, is_sin ? ms : m, false);
+        const double f = twiddle_flip(sm2, D, is_sin ? m : ms, neg);
+        acc = fma(t, v[i].x, acc);
+        acc2 = fma(f, v[i].y, acc2);
+        m += inc;
+        if (m >= D4) m -= D4;
       }
     }
   }
+  acc += acc2;
 #pragma unroll
   for (int off = KO; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (lane < KO) red[warp][lane] = acc;
@@ -1494,7 +1505,8 @@ void pick_factors(int D, int nin, int nout, int* Aout, int* Bout) {
   for (int A = 2; A <= D / 2; ++A) {
     if (D % A) continue;
     const int B = D / A;
-    if (B < 2 || B > 256) continue;  // pass 2 stages B x 32 twiddle pairs
+    if (B < 2 || B > 256) continue;  // pass 2 of many lines stages B x 32 twiddle pairs
+    if (32LL * A + 16LL * (A + 2) > 180 * 1024) continue;  // pass 1's table and inputs
     const double cost = x_two_level_cost(A, B, D, nin, nout);
     if (cost < best) {
       best = cost;
@@ -1532,10 +1544,11 @@ int p1_terms(const AxisJob& J) { return (std::min(J.jhi, J.nin) + J.B - 1) / J.B
 // Shared memory of the passes (the twiddles, pass 1 also the inputs).
 size_t pass1_smem(const AxisJob& J, int P) {
   const int K = p1_terms(J), Kp = (K + 1) & ~1;
-  const P1Shape s = p1_shape(J.A, J.B, K, P);
-  return sizeof(double) * ((size_t)Kp * s.nk * 2 + (size_t)Kp * s.G);
+  const P1Shape s = p1_shape(J.A, J.B, P);
+  return sizeof(double) * (4 * (size_t)J.A + (size_t)Kp * s.G);
 }
-size_t pass2_smem(const AxisJob& J, int KO) { return sizeof(double) * 2 * KO * (size_t)J.B; }
+size_t pass2_smem(const AxisJob& J) { return sizeof(double) * ((size_t)J.D + 1); }
+size_t pass2_lines_smem(const AxisJob& J) { return sizeof(double) * 2 * 32 * (size_t)J.B; }
 
 // FMAs of a two-level pass pair on one line
 double two_level_fmas(const AxisJob& J) {
@@ -1573,7 +1586,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     long long n = 0;
     for (int i = 0; i < b.njobs; ++i) {
       const AxisJob& J = b.job[i];
-      const P1Shape s = p1_shape(J.A, J.B, p1_terms(J), P);
+      const P1Shape s = p1_shape(J.A, J.B, P);
       n += (long long)J.nlines * s.kblocks * s.jblocks;
     }
     return n;
@@ -1584,7 +1597,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
     const AxisJob& J = b.job[i];
-    const P1Shape s = p1_shape(J.A, J.B, p1_terms(J), P);
+    const P1Shape s = p1_shape(J.A, J.B, P);
     smem1 = std::max(smem1, pass1_smem(J, P));
     b.start[i] = total;
     total += J.nlines * s.kblocks * s.jblocks;
@@ -1611,7 +1624,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     for (int i = 0; i < b.njobs; ++i) {
       b.start[i] = total;
       total += ((b.job[i].nlines + lpc - 1) / lpc) * ((p2_lanes(b.job[i]) + 31) / 32);
-      smem2 = std::max(smem2, pass2_smem(b.job[i], 32));
+      smem2 = std::max(smem2, pass2_lines_smem(b.job[i]));
     }
     b.start[b.njobs] = total;
     with_capacity(b.njobs, [&](auto c) {
@@ -1632,7 +1645,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   for (int i = 0; i < b.njobs; ++i) {
     b.start[i] = total;
     total += b.job[i].nlines * ((p2_lanes(b.job[i]) + KO - 1) / KO);
-    smem2 = std::max(smem2, pass2_smem(b.job[i], KO));
+    smem2 = std::max(smem2, pass2_smem(b.job[i]));
   }
   b.start[b.njobs] = total;
   if (total > 0)
