@@ -2,18 +2,28 @@
 //
 //   D[m, n] = act( sum_k A[m, k] B[n, k] + bias[n] )      (FP32 accumulate)
 //
-// A (M x K) and B (N x K) are BF16, row-major with K contiguous ("K-major"
-// for both operands); D is FP32 or BF16, row-major with leading dimension
-// ldd.  One CTA computes one 128 x BN tile:
-//   - warp 0, one thread: TMA loads of 128 x 64 A and BN x 64 B tiles
+// A (M x K) and B (N x K) are BF16, each row-major with K contiguous ("K-major")
+// or with M (N) contiguous (a transposed view, "MN-major", read as it lies);
+// D is FP32 or BF16, row-major with leading dimension ldd.  One CTA computes one
+// 128 x BN tile:
+//   - warp 0, one elected lane: TMA loads of the 128 x 64 A and BN x 64 B tiles
 //     (128-byte swizzle) into a kStages-deep shared-memory ring, each stage
 //     signalled on an mbarrier with its byte count;
-//   - warp 1, one thread: tcgen05.mma (kind::f16, BF16 inputs, FP32
+//   - warp 1, one elected lane: tcgen05.mma (kind::f16, BF16 inputs, FP32
 //     accumulator in tensor memory), four K=16 steps per stage; a
 //     tcgen05.commit per stage frees the stage for the next TMA load, and a
 //     last commit signals the epilogue;
-//   - all four warps: tcgen05.ld of their 32 accumulator lanes, bias and
-//     activation, stores.
+//   - all eight warps: tcgen05.ld of their 32 accumulator lanes (two warps per
+//     32 lanes, half of the columns each), bias and activation, stores.
+// A product of few tiles and many terms (a truncated transform of 2052 points, the
+// weight gradients of small batches) is cut along K (split_count): every slice
+// writes its FP32 sums to the caller's workspace and k_tc_reduce adds them in a
+// fixed order.
+// Measured (with views read in place, before -> now, a call alone): 65664 x 32 over
+// 32 modes of a grid 42 -> 37 us, the larger drawn contractions 105 -> 68 us;
+// kernel only: 32 x 32 over 65664 terms 299 -> 150 us, over 6144 33 -> 21 us,
+// 8192^3 1.29 -> 1.19 ms.  A single tile over many terms is bound by the latency of
+// the ring (about 280 cycles for a stage of 64 terms), a narrow product by memory.
 // Every wait on an mbarrier is bounded: on timeout the CTA records an error
 // code in a device flag, skips its remaining work, frees its tensor memory
 // and returns.
@@ -21,8 +31,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "hosnwt_internal.h"
 
@@ -31,8 +44,12 @@ namespace {
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;         // one 128-byte swizzle atom of BF16
-constexpr int kStages = 4;
-constexpr int kThreads = 128;
+// stages of the ring: 4 let two CTAs share an SM; where every CTA has an SM of
+// its own the ring takes what fits
+constexpr int kStagesFew = 4;
+template <int BN>
+constexpr int kStagesDeep = BN > 64 ? 6 : 8;
+constexpr int kThreads = 256;
 constexpr unsigned kSpinLimit = 1u << 22;  // try_wait polls (each may suspend briefly): seconds at most
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
@@ -43,9 +60,27 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
+// The loops that load and that issue run in a converged warp, one elected lane
+// acting by a predicate on the instruction, so that addresses and descriptors stay
+// in uniform registers (one thread in a branch took 560 cycles for a stage of a
+// single tile, this 280).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e;
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(bytes), "r"(elected)
+      : "memory");
 }
 
 // Wait for the phase of the given parity to complete; false on timeout.
@@ -65,11 +100,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   return false;
 }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar,
+                                            uint32_t elected) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::
+          "r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "r"(elected)
       : "memory");
 }
 
@@ -88,24 +126,39 @@ __device__ __forceinline__ uint64_t sw128_desc(unsigned saddr) {
   return d;
 }
 
-// Instruction descriptor: FP32 accumulator, BF16 A and B, both K-major,
-// N = bn, M = 128.
-__host__ __device__ constexpr uint32_t idesc_bf16(int bn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+// The same of an MN-major tile: blocks of 64 elements of M (or N) by kBK rows of
+// K, rows of 128 bytes, 8-row groups 1024 bytes apart (SBO), blocks
+// kBK * 128 bytes apart (LBO); a K=16 slice is 16 rows, 2048 bytes.
+__device__ __forceinline__ uint64_t sw128_desc_mn(unsigned saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((kBK * 128) >> 4) << 16) |
+         ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, int accumulate) {
+// Instruction descriptor: FP32 accumulator, BF16 A and B, K-major or MN-major
+// (bits 15, 16), N = bn, M = 128.
+__host__ __device__ constexpr uint32_t idesc_bf16(int bn, bool ta, bool tb) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (ta ? 1u << 15 : 0u) | (tb ? 1u << 16 : 0u) |
+         ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, int accumulate,
+                                         uint32_t elected) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void mma_commit(uint64_t* bar, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+      "r"(elected)
+      : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
@@ -135,19 +188,54 @@ struct GemmArgs {
   const float* bias;   // N entries or null
   int act;             // 0 none, 1 GELU
   const float* Dadd;   // optional FP32 M x N (ldd) added before the activation
+  int kb_per;          // stages per slice of K
+  int rows_a, rows_b;  // rows of a K-major box: the tile's, but no more than the matrix has
+                       // also where it lies outside the matrix
+  float* part;         // slices > 1: FP32 sums [slice][M][N], else null
   unsigned* err;       // error flag (1: a wait timed out; 2: the wait for the
                        // MMAs to finish timed out too, so the CTA exited
                        // without freeing its tensor memory: treat the
                        // context as unusable)
 };
 
-template <int BN>
+__device__ __forceinline__ void store_out(const GemmArgs& g, int row, int col, float x) {
+  const long long o = (long long)row * g.ldd + col;
+  if (g.Dadd) x += g.Dadd[o];
+  if (g.act == 1) x = gelu(x);
+  if (g.d_bf16)
+    ((__nv_bfloat16*)g.D)[o] = __float2bfloat16(x);
+  else
+    ((float*)g.D)[o] = x;
+}
+
+// D from the slices' sums: 32 outputs per block, 8 warps over the slices
+__global__ void __launch_bounds__(256) k_tc_reduce(GemmArgs g, int slices) {
+  __shared__ float red[8][32];
+  const long long n = (long long)g.M * g.N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long i = blockIdx.x * 32LL + lane;
+  float x = 0.0f;
+  if (i < n)
+#pragma unroll 4
+    for (int s = warp; s < slices; s += 8) x += __ldcg(g.part + s * n + i);
+  red[warp][lane] = x;
+  __syncthreads();
+  if (warp == 0 && i < n) {
+    const float y = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) +
+                    ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
+    const int row = (int)(i / g.N), col = (int)(i - (long long)row * g.N);
+    store_out(g, row, col, y + (g.bias ? g.bias[col] : 0.0f));
+  }
+}
+
+template <int BN, bool TA, bool TB, int kStages>
 __global__ void __launch_bounds__(kThreads, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, GemmArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // 1024-byte aligned stage ring: kStages x (A 128x64, B BNx64) BF16
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int kABytes = kBM * kBK * 2, kBBytes = BN * kBK * 2;
+  constexpr int kBRows = TB && BN < 64 ? 64 : BN;  // an MN-major block is 64 wide
+  constexpr int kABytes = kBM * kBK * 2, kBBytes = kBRows * kBK * 2;
   unsigned char* sA = base;
   unsigned char* sB = base + kStages * kABytes;
   __shared__ uint64_t full_bar[kStages], empty_bar[kStages], done_bar;
@@ -157,7 +245,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ int n_issued, n_consumed;  // stages loaded by TMA / read by the MMAs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-  const int nk = (g.K + kBK - 1) / kBK;
+  const int kb0 = blockIdx.z * g.kb_per;
+  const int nk = min((g.K + kBK - 1) / kBK - kb0, g.kb_per);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -182,22 +271,38 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
 
-  if (warp == 0 && lane == 0) {
-    // producer
+  if (warp == 0) {
+    const uint32_t elected = elect_one();
+    // producer: 64-wide blocks of an MN-major operand, or one box of its rows
+    const int blk_a = min(kBM, g.M - m0 + 63) / 64, blk_b = min(kBRows, g.N - n0 + 63) / 64;
+    const unsigned bytes_a = TA ? blk_a * (kBK * 128) : g.rows_a * 128;
+    const unsigned bytes_b = TB ? blk_b * (kBK * 128) : g.rows_b * 128;
     for (int kb = 0; kb < nk; ++kb) {
       const int s = kb % kStages, r = kb / kStages;
       if (kb >= kStages && !mbar_wait(&empty_bar[s], (unsigned)((r - 1) & 1))) {
         abort_flag = 1;
         break;
       }
-      mbar_expect_tx(&full_bar[s], kABytes + kBBytes);
-      tma_load_2d(sA + s * kABytes, &mapA, kb * kBK, m0, &full_bar[s]);
-      tma_load_2d(sB + s * kBBytes, &mapB, kb * kBK, n0, &full_bar[s]);
-      n_issued = kb + 1;
+      mbar_expect_tx(&full_bar[s], bytes_a + bytes_b, elected);
+      const int k0 = (kb0 + kb) * kBK;
+      if constexpr (TA) {
+        for (int q = 0; q < blk_a; ++q)
+          tma_load_2d(sA + s * kABytes + q * (kBK * 128), &mapA, m0 + 64 * q, k0, &full_bar[s], elected);
+      } else {
+        tma_load_2d(sA + s * kABytes, &mapA, k0, m0, &full_bar[s], elected);
+      }
+      if constexpr (TB) {
+        for (int q = 0; q < blk_b; ++q)
+          tma_load_2d(sB + s * kBBytes + q * (kBK * 128), &mapB, n0 + 64 * q, k0, &full_bar[s], elected);
+      } else {
+        tma_load_2d(sB + s * kBBytes, &mapB, k0, n0, &full_bar[s], elected);
+      }
+      if (elected) n_issued = kb + 1;
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
+    const uint32_t elected = elect_one();
     // MMA issuer
-    constexpr uint32_t idesc = idesc_bf16(BN);
+    constexpr uint32_t idesc = idesc_bf16(BN, TA, TB);
     bool ok = true;
     for (int kb = 0; kb < nk; ++kb) {
       const int s = kb % kStages, r = kb / kStages;
@@ -206,16 +311,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t da = sw128_desc(smem_u32(sA + s * kABytes));
-      const uint64_t db = sw128_desc(smem_u32(sB + s * kBBytes));
+      const uint64_t da = TA ? sw128_desc_mn(smem_u32(sA + s * kABytes)) : sw128_desc(smem_u32(sA + s * kABytes));
+      const uint64_t db = TB ? sw128_desc_mn(smem_u32(sB + s * kBBytes)) : sw128_desc(smem_u32(sB + s * kBBytes));
 #pragma unroll
       for (int kk = 0; kk < kBK / 16; ++kk)
-        mma_bf16(tmem, da + 2 * kk, db + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1 : 0);
-      mma_commit(&empty_bar[s]);
-      n_consumed = kb + 1;
+        mma_bf16(tmem, da + (TA ? 128 : 2) * kk, db + (TB ? 128 : 2) * kk, idesc, (kb > 0 || kk > 0) ? 1 : 0, elected);
+      mma_commit(&empty_bar[s], elected);
+      if (elected) n_consumed = kb + 1;
     }
     if (!ok) abort_flag = 1;
-    mma_commit(&done_bar);  // arrives once every MMA issued above has completed
+    mma_commit(&done_bar, elected);  // arrives once every MMA issued above has completed
   }
   __syncwarp();
   // epilogue: every warp waits for the accumulator
@@ -243,10 +348,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     // reads, combines and stores 16 consecutive columns of one row.
     float* tile = reinterpret_cast<float*>(base) + warp * (32 * 17);
     const int half = lane >> 4, cl = lane & 15;
+    const int quad = warp & 3;
+    constexpr int kCols = BN / 2;  // of each of the two warps of 32 rows
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
+    for (int c0 = (warp >> 2) * kCols; c0 < ((warp >> 2) + 1) * kCols; c0 += 16) {
       float v[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) tile[lane * 17 + i] = v[i];
       __syncwarp();
@@ -254,15 +361,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float bcol = (g.bias && col < g.N) ? g.bias[col] : 0.0f;
 #pragma unroll 4
       for (int r = half; r < 32; r += 2) {
-        const int row = m0 + warp * 32 + r;
+        const int row = m0 + quad * 32 + r;
         if (row < g.M && col < g.N) {
-          float x = tile[r * 17 + cl] + bcol;
-          if (g.Dadd) x += g.Dadd[(long long)row * g.ldd + col];
-          if (g.act == 1) x = gelu(x);
-          if (g.d_bf16)
-            ((__nv_bfloat16*)g.D)[(long long)row * g.ldd + col] = __float2bfloat16(x);
-          else
-            ((float*)g.D)[(long long)row * g.ldd + col] = x;
+          float x = tile[r * 17 + cl];
+          if (g.part) {
+            g.part[((long long)blockIdx.z * g.M + row) * g.N + col] = x;
+          } else {
+            x += bcol;
+            store_out(g, row, col, x);
+          }
         }
       }
       __syncwarp();
@@ -305,45 +412,126 @@ bool make_map(CUtensorMap* m, const void* ptr, int rows, int cols, long long ld,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
-cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, cudaStream_t st) {
-  const size_t smem = 1024 + (size_t)kStages * (kBM + BN) * kBK * 2;
+int sm_count() {
+  static std::atomic<int> nsm[256];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) return 1;
+  int v = nsm[dev].load(std::memory_order_relaxed);
+  if (v == 0) {
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 1;
+    nsm[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
+
+template <int BN, bool TA, bool TB, int kStages>
+cudaError_t launch_ring(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, dim3 grid, cudaStream_t st) {
+  constexpr int kBRows = TB && BN < 64 ? 64 : BN;
+  const size_t smem = 1024 + (size_t)kStages * (kBM + kBRows) * kBK * 2;
   static PerDeviceOnce attr;
-  attr.run([&] { cudaFuncSetAttribute(k_tc_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-  const dim3 grid((g.M + kBM - 1) / kBM, (g.N + BN - 1) / BN);
-  k_tc_gemm<BN><<<grid, kThreads, smem, st>>>(ma, mb, g);
+  attr.run([&] {
+    cudaFuncSetAttribute(k_tc_gemm<BN, TA, TB, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  k_tc_gemm<BN, TA, TB, kStages><<<grid, kThreads, smem, st>>>(ma, mb, g);
   return cudaGetLastError();
+}
+
+template <int BN, bool TA, bool TB>
+cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, int slices, cudaStream_t st) {
+  const dim3 grid((g.M + kBM - 1) / kBM, (g.N + BN - 1) / BN, slices);
+  if ((long long)grid.x * grid.y * grid.z <= sm_count())
+    return launch_ring<BN, TA, TB, kStagesDeep<BN>>(ma, mb, g, grid, st);
+  return launch_ring<BN, TA, TB, kStagesFew>(ma, mb, g, grid, st);
+}
+
+int tile_cols(int N) { return N <= 32 ? 32 : (N <= 64 ? 64 : 128); }
+
+// Slices of K: where the tiles leave most SMs idle and a slice keeps four
+// stages (a slice costs its 4 bytes per output twice, and the reduction a
+// launch of 3 us; below 16 stages the product itself takes less).  Sums longer than
+// 6144 terms stay whole: their FP32 accumulation is off by up to 8e-5 of the
+// result, and a call keeps the value that one accumulator gives.
+int split_count(int M, int N, int K) {
+  const int nsm = sm_count(), bn = tile_cols(N);
+  const long long tiles = ((long long)M + kBM - 1) / kBM * ((N + bn - 1) / bn);
+  const int kb = (K + kBK - 1) / kBK;
+  if (kb < 16 || K > 6144 || 2 * tiles > nsm) return 1;
+  const int want = (int)std::min<long long>(nsm / tiles, kb / 4);
+  if (want < 2) return 1;
+  const int per = (kb + want - 1) / want;
+  return (kb + per - 1) / per;
 }
 
 }  // namespace
 
-// D = act(A B^T + bias [+ Dadd]); see the file comment.  A: M x K (lda),
-// B: N x K (ldb), both BF16; K, lda, ldb multiples of 8 and both base
-// addresses 16-byte aligned (the TMA rules).  Returns a cudaError_t value
-// (cudaErrorInvalidValue for shapes the kernel does not take).
-int tc_gemm_bf16(const void* A, long long lda, const void* B, long long ldb, void* D, long long ldd, int d_bf16,
-                 int M, int N, int K, const float* bias, int act, const float* Dadd, unsigned* err,
-                 cudaStream_t st) {
-  if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (lda % 8) || (ldb % 8) || ((uintptr_t)A & 15) ||
+// D = act(A B^T + bias [+ Dadd]); see the file comment.  A: M x K with row
+// stride lda, or its transpose K x M (ta); B: N x K, or K x N (tb), both BF16;
+// lda and ldb multiples of 8, K a multiple of 8 where an operand has it
+// contiguous, both base addresses 16-byte aligned (the TMA rules).  work holds
+// split_count(M, N, K) * M * N floats where that count is above one (else, or
+// null, K is not cut).  Returns a cudaError_t value (cudaErrorInvalidValue for
+// shapes the kernel does not take).
+int tc_gemm_bf16(const void* A, long long lda, bool ta, const void* B, long long ldb, bool tb, void* D, long long ldd,
+                 int d_bf16, int M, int N, int K, const float* bias, int act, const float* Dadd, float* work,
+                 unsigned* err, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || K <= 0 || (!(ta && tb) && (K % 8)) || (lda % 8) || (ldb % 8) || ((uintptr_t)A & 15) ||
       ((uintptr_t)B & 15) || !err)
     return (int)cudaErrorInvalidValue;
-  const int bn = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  const int bn = tile_cols(N);
   CUtensorMap ma, mb;
-  if (!make_map(&ma, A, M, K, lda, kBM) || !make_map(&mb, B, N, K, ldb, bn)) return (int)cudaErrorInvalidValue;
-  GemmArgs g{M, N, K, D, ldd, d_bf16, bias, act, Dadd, err};
-  cudaError_t e;
-  if (bn == 32) e = launch_gemm<32>(ma, mb, g, st);
-  else if (bn == 64) e = launch_gemm<64>(ma, mb, g, st);
-  else e = launch_gemm<128>(ma, mb, g, st);
+  // boxes no higher than the matrix (whole 8-row swizzle groups): the accumulator
+  // rows and columns beyond it take what the shared memory holds, and are dropped
+  const int rows_a = std::min(kBM, (M + 7) / 8 * 8), rows_b = std::min(bn, (N + 7) / 8 * 8);
+  if (!(ta ? make_map(&ma, A, K, M, lda, kBK) : make_map(&ma, A, M, K, lda, rows_a)) ||
+      !(tb ? make_map(&mb, B, K, N, ldb, kBK) : make_map(&mb, B, N, K, ldb, rows_b)))
+    return (int)cudaErrorInvalidValue;
+  const int kb = (K + kBK - 1) / kBK;
+  const int slices = work ? split_count(M, N, K) : 1;
+  GemmArgs g{M, N, K, D, ldd, d_bf16, bias, act, Dadd, (kb + slices - 1) / slices, rows_a, rows_b,
+             slices > 1 ? work : nullptr, err};
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto bnc) {
+    constexpr int BN = decltype(bnc)::value;
+    if (ta && tb) e = launch_gemm<BN, true, true>(ma, mb, g, slices, st);
+    else if (ta) e = launch_gemm<BN, true, false>(ma, mb, g, slices, st);
+    else if (tb) e = launch_gemm<BN, false, true>(ma, mb, g, slices, st);
+    else e = launch_gemm<BN, false, false>(ma, mb, g, slices, st);
+  };
+  if (bn == 32) go(std::integral_constant<int, 32>());
+  else if (bn == 64) go(std::integral_constant<int, 64>());
+  else go(std::integral_constant<int, 128>());
+  if (e == cudaSuccess && slices > 1) {
+    const long long n = (long long)M * N;
+    k_tc_reduce<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(g, slices);
+    e = cudaGetLastError();
+  }
   return (int)e;
 }
 
 }  // namespace hos
 
+static int gemm_status(int e) {
+  return e == 0 ? HOSNWT_OK : (e == (int)cudaErrorInvalidValue ? HOSNWT_ERR_ARG : HOSNWT_ERR_CUDA);
+}
+
 extern "C" int hosnwt_tc_gemm_bf16(const void* A, long long lda, const void* B, long long ldb, void* D,
                                    long long ldd, int d_bf16, int M, int N, int K, const float* bias, int act,
                                    const float* Dadd, unsigned* err, void* stream) {
-  const int e = hos::tc_gemm_bf16(A, lda, B, ldb, D, ldd, d_bf16, M, N, K, bias, act, Dadd, err,
-                                  (cudaStream_t)stream);
-  return e == 0 ? HOSNWT_OK : (e == (int)cudaErrorInvalidValue ? HOSNWT_ERR_ARG : HOSNWT_ERR_CUDA);
+  return gemm_status(hos::tc_gemm_bf16(A, lda, false, B, ldb, false, D, ldd, d_bf16, M, N, K, bias, act, Dadd, nullptr,
+                                       err, (cudaStream_t)stream));
+}
+
+extern "C" long long hosnwt_tc_gemm_workspace(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int s = hos::split_count(M, N, K);
+  return s > 1 ? 4LL * s * M * N : 0;
+}
+
+extern "C" int hosnwt_tc_gemm_bf16_ex(const void* A, long long lda, int ta, const void* B, long long ldb, int tb,
+                                      void* D, long long ldd, int d_bf16, int M, int N, int K, const float* bias,
+                                      int act, const float* Dadd, void* work, long long work_bytes, unsigned* err,
+                                      void* stream) {
+  if (work && work_bytes < hosnwt_tc_gemm_workspace(M, N, K)) return HOSNWT_ERR_ARG;
+  return gemm_status(hos::tc_gemm_bf16(A, lda, ta != 0, B, ldb, tb != 0, D, ldd, d_bf16, M, N, K, bias, act, Dadd,
+                                       (float*)work, err, (cudaStream_t)stream));
 }

@@ -47,24 +47,51 @@ def _err_flag(device):
     return _ERR[key]
 
 
+# Contractions over more terms than this read their operands with the terms
+# contiguous: they run on one tile, bound by the time of a 64-term stage, which
+# for a narrow transposed operand takes 64 rows of a TMA load and for a copied
+# one as many as it has rows (16 channels, 2 blocks, backward included: 0.48 ms
+# with the copies, 0.55 ms in place).
+_LONG_K = 6144
+
+
+def _operand(t, in_place):
+    """(tensor, transposed) that the kernel can read as it lies: rows
+    contiguous, 16-byte aligned, a row stride of whole 16 bytes; a transposed
+    view is handed over as the matrix under it (`in_place`), anything else is
+    copied, with the row zero-padded to a multiple of 8."""
+    torch = _torch()
+    r, c = t.shape
+    s0, s1 = t.stride()
+    if t.data_ptr() % 16 == 0:
+        if s1 == 1 and c % 8 == 0 and (s0 % 8 == 0 and s0 >= c or r == 1):
+            return t, False
+        if in_place and s0 == 1 and s1 % 8 == 0 and s1 >= r and c > 1:
+            return t.t(), True
+    if c % 8:
+        t = torch.nn.functional.pad(t, (0, 8 - c % 8))
+    t = t.contiguous()
+    return (t.clone() if t.data_ptr() % 16 else t), False
+
+
 def gemm_bf16(A, B):
     """D = A B^T on tcgen05: A (R, K), B (N, K) cast to BF16; D FP32 (R, N).
-    K is zero-padded to a multiple of 8 (the TMA row-stride rule)."""
+    Transposed views are read in place; K is zero-padded to a multiple of 8
+    where an operand has it contiguous (the TMA row-stride rule)."""
     torch = _torch()
-    A = A.to(torch.bfloat16)
-    B = B.to(torch.bfloat16)
-    K = A.shape[1]
-    if K % 8:
-        pad = 8 - K % 8
-        A = torch.nn.functional.pad(A, (0, pad))
-        B = torch.nn.functional.pad(B, (0, pad))
-    A = A.contiguous()
-    B = B.contiguous()
-    if A.data_ptr() % 16:
-        A = A.clone()
-    if B.data_ptr() % 16:
-        B = B.clone()
-    return hosnwt.tc_gemm(A, B, err=_err_flag(A.device), stream=torch.cuda.current_stream().cuda_stream)
+    A = A if A.dtype == torch.bfloat16 else A.to(torch.bfloat16)
+    B = B if B.dtype == torch.bfloat16 else B.to(torch.bfloat16)
+    M, K = A.shape
+    N = B.shape[0]
+    a, ta = _operand(A, K <= _LONG_K)
+    b, tb = _operand(B, K <= _LONG_K)
+    if ta != tb and K % 8:
+        # the padded row of one operand would meet the K rows of the other
+        a, ta = _operand(A, False)
+        b, tb = _operand(B, False)
+    out = torch.empty((M, N), dtype=torch.float32, device=A.device)
+    st = torch.cuda.current_stream(A.device).cuda_stream
+    return hosnwt.tc_gemm_views(a, b, ta, tb, None, 0, None, out, _err_flag(A.device), st, st)
 
 
 def check_kernel_flags():
