@@ -16,9 +16,9 @@
 // 0, 1, 2, 3, and one for the levels 4 and 5.  A sum of level 0 to 3 is a whole
 // number below 2^24 units over 128 (levels 0, 1) or 64 terms (2, 3), so every
 // addition is exact; then it is added to a 64-bit fixed-point sum (34
-// fractional bits), which is exact too: a result does not depend on the order
-// or the split of the work.  In the fifth accumulator the FP32 rounding is 2^-24
-// of products below 2^-36 of the largest.  What is left out (level 6 and the
+// fractional bits), which is exact too.  In the fifth accumulator the FP32 rounding is 2^-24 of
+// products below 2^-36 of the largest: all that a result owes to the order and
+// the split of the work.  What is left out (level 6 and the
 // remainders of the sixth digits) is 2^-54 of the largest product per term.
 //
 // Half of the work is saved by one fold per pass:
@@ -166,18 +166,22 @@ __device__ __forceinline__ uint64_t sw64_desc(unsigned saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
 }
-// FP32 accumulator, BF16 operands, both K-major, N = kBN, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+// FP32 accumulator, BF16 operands, both K-major, M = 128
+constexpr uint32_t idesc_of(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
+constexpr uint32_t kIdesc = idesc_of(kBN), kIdescWide = idesc_of(2 * kBN);
 
 // Issued by the elected lane of a converged warp: the branch stays inside
 // the instruction, so that the descriptors live in uniform registers.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, int accumulate, uint32_t elected) {
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, int accumulate,
+                                         uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "setp.ne.b32 q, %5, 0;\n\t"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate), "r"(elected)
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar, uint32_t elected) {
@@ -500,11 +504,19 @@ __global__ void __launch_bounds__(kDgThreads) k_tc_digits_y(const __grid_constan
 
 // ---------------------------------------------------------------- the product
 
-// pairs (i, j) of digits: levels 5 and 4 (accumulator 4), then 0, 1, 2, 3
-constexpr int kLow = 11, kMid = kLow + 3, kPairs = kMid + 7;
-__device__ constexpr signed char kPairI[kPairs] = {0, 5, 1, 4, 2, 3, 0, 4, 1, 3, 2, 0, 0, 1, 0, 2, 1, 0, 3, 1, 2};
-__device__ constexpr signed char kPairJ[kPairs] = {5, 0, 4, 1, 3, 2, 4, 0, 3, 1, 2, 0, 1, 0, 2, 0, 1, 3, 0, 2, 1};
-__device__ constexpr signed char kPairG[kPairs] = {4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 0, 1, 1, 2, 2, 2, 3, 3, 3, 3};
+// The 21 pairs (i, j) of digits.  Twelve are issued two at a time: digits j and
+// j + 1 of the matrix are neighbours in shared memory and the accumulators of
+// levels i + j and i + j + 1 neighbours in tensor memory, so one instruction of
+// 192 columns takes digit i of the lines against both and reads it once.  The
+// other nine go to accumulator 4, the smallest first.  What bounds the products
+// is the tensor cores' sustained rate: 2850 cycles per stage are 1.8 PFLOP/s in
+// BF16 (1.2 kW at 2070 MHz), with 21 narrow products 2900; a time step of 2052 x
+// 1028 modes at order 9, 193.7 -> 190.2 ms.
+constexpr int kNarrow = 9, kWide = 6;
+__device__ constexpr signed char kNarrowI[kNarrow] = {0, 5, 1, 4, 2, 3, 0, 4, 2};
+__device__ constexpr signed char kNarrowJ[kNarrow] = {5, 0, 4, 1, 3, 2, 4, 0, 2};
+__device__ constexpr signed char kWideI[kWide] = {0, 0, 1, 2, 1, 3};
+__device__ constexpr signed char kWideJ[kWide] = {0, 2, 0, 0, 2, 0};
 
 // a 2^e, rounded to nearest, by integer arithmetic: conversions and products
 // in FP64 cost 64 issue cycles of a warp each.  -1000 < e < 900
@@ -786,27 +798,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
             }
             const unsigned sa = smem_u32(base) + s * kStageBytes;
             const uint64_t da = sw64_desc(sa), db = sw64_desc(sa + kABytes);
-            auto product = [&](int q, bool fresh) {
+            auto product = [&](int i, int j, int g, uint32_t idesc, bool fresh) {
 #pragma unroll
               for (int kk = 0; kk < 2; ++kk)
-                mma_bf16(tmem + kPairG[q] * kBN, da + kPairI[q] * (kBM * kBK * 2 / 16) + 2 * kk,
-                         db + kPairJ[q] * (kBN * kBK * 2 / 16) + 2 * kk,
-                         !(fresh && kk == 0 && (q == 0 || kPairG[q] != kPairG[q - 1])), elected);
+                mma_bf16(tmem + g * kBN, da + i * (kBM * kBK * 2 / 16) + 2 * kk,
+                         db + j * (kBN * kBK * 2 / 16) + 2 * kk, idesc, !(fresh && kk == 0), elected);
+            };
+            auto wide = [&](int q, bool fresh) {
+              product(kWideI[q], kWideJ[q], kWideI[q] + kWideJ[q], kIdescWide, fresh);
             };
             if (kb == 0 && !wait_drained(2)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int q = 0; q < kLow; ++q) product(q, kb == 0);
+            for (int q = 0; q < kNarrow; ++q) product(kNarrowI[q], kNarrowJ[q], 4, kIdesc, kb == 0 && q == 0);
             if (hi0 && !wait_drained(0)) break;
-#pragma unroll
-            for (int q = kLow; q < kMid; ++q) product(q, hi0);
+            wide(0, hi0);
+            if (lo0 && !wait_drained(1)) break;
+            wide(1, lo0);
+            wide(2, false);
             if (hi1) {
               mma_commit(&acc_full[0], elected);
               ++nd[0];
             }
-            if (lo0 && !wait_drained(1)) break;
 #pragma unroll
-            for (int q = kMid; q < kPairs; ++q) product(q, lo0);
+            for (int q = 3; q < kWide; ++q) wide(q, false);
             if (lo1) {
               mma_commit(&acc_full[1], elected);
               ++nd[1];
