@@ -72,27 +72,6 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// The same with a thread-block cluster of `cluster` CTAs along x.
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                      int cluster, cudaStream_t st, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = g_launch_no_pdl ? attr + 1 : attr;
-  cfg.numAttrs = g_launch_no_pdl ? 1 : 2;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // ---------------------------------------------------------------------------
 // Spectral transforms along one axis.
 //
@@ -394,7 +373,8 @@ void launch_fft_jobs(const AxisBatch& b, const FftPlanInfo* const* plan, const T
 // pass alone (npass = 1).  launch_tc_jobs runs the jobs of a batch (all x or
 // all y passes, every one with its matrix), false if one of them does not fit
 // the scratch.
-bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<void*>& allocs, TcMat* out);
+bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<long double>& quarter,
+                     double* scratch, std::vector<void*>& allocs, TcMat* out);
 // Scratch (doubles) that holds the digits of `first` lines of `second` points
 // for each of the given pairs, one at a time.
 long long tc_scratch_doubles(int nsm, const std::vector<std::pair<long long, int>>& lines);

@@ -870,12 +870,14 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
   // also truncated to the free-surface modes
   c.tb.ntc = 0;
   if (n2 > 1) {
+    std::vector<long double> quarter;
+    double* const tmp = c.tb.cs ? c.tb.cs + kTcMaxBytes / 8 : nullptr;  // behind the maxima and the error flag
     auto add = [&](int D, int form, int sin_kind, double scale, int nout) {
       for (int i = 0; i < c.tb.ntc; ++i) {
         const TcMat& m = c.tb.tc[i];
         if (m.D == D && m.form == form && m.sin_kind == sin_kind && m.scale == scale && nout <= m.nout) return;
       }
-      if (c.tb.ntc < kTcMats && build_tc_matrix(D, form, sin_kind, scale, nout, c.allocs, &c.tb.tc[c.tb.ntc])) ++c.tb.ntc;
+      if (c.tb.ntc < kTcMats && build_tc_matrix(D, form, sin_kind, scale, nout, quarter, tmp, c.allocs, &c.tb.tc[c.tb.ntc])) ++c.tb.ntc;
     };
     for (int axis = 0; axis < 2; ++axis) {
       const int n = axis ? n2 : n1, nd = axis ? nd2 : nd1;
@@ -886,6 +888,7 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
       }
       if (nd > n) add(nd - 1, 1, 0, 2.0 * (1.0 / (nd - 1)), n);
     }
+    if (cudaStreamSynchronize(0) != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "transform matrices failed");
   }
   for (Tables* t : {&c.tb2, &c.tb3}) {
     t->ntc = c.tb.ntc;

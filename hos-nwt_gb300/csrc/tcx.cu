@@ -1116,12 +1116,17 @@ int tc_mode() {
 }  // namespace
 
 // The matrix of one form of a pass of length D (see TcMat).  scale is the
-// interior output scale times the interior input weight.
-bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<void*>& allocs, TcMat* out) {
-  if (D < 8 || D > kTcMaxD) return false;
+// interior output scale times the interior input weight; quarter holds the first
+// quarter turn's cosines, filled as they are asked for (the forms of a length
+// share them); the table of entries passes through `scratch`.  The matrix is
+// complete once the default stream is.
+bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<long double>& quarter,
+                     double* scratch, std::vector<void*>& allocs, TcMat* out) {
+  if (D < 8 || D > kTcMaxD || !scratch) return false;
   int ew = 0;
   const long double c = frexpl((long double)scale, &ew);  // scale = c 2^ew, c in [1/2, 1)
   const long double pi = 3.141592653589793238462643383279502884L;
+  if ((int)quarter.size() != D + 1) quarter.assign(D + 1, 2.0L);
   std::vector<unsigned short> tab((size_t)2 * D * 8, 0);
   for (int q = 0; q < 2 * D; ++q) {
     // cos(pi m / (2 D)) with the angle folded to the first quarter turn
@@ -1130,34 +1135,27 @@ bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std:
     if (m > 2 * D) m = 4 * D - m;
     const bool neg = m > D;
     if (neg) m = 2 * D - m;
-    long double v = (m == D) ? 0.0L : (2 * m > D ? sinl(pi * (long double)(D - m) / (2.0L * D))
-                                                 : cosl(pi * (long double)m / (2.0L * D)));
-    v *= neg ? -c : c;
+    long double& v = quarter[m];
+    if (v > 1.0L)
+      v = (m == D) ? 0.0L
+                   : (2 * m > D ? sinl(pi * (long double)(D - m) / (2.0L * D)) : cosl(pi * (long double)m / (2.0L * D)));
     float d[5];
-    split_digits(llrintl(ldexpl(v, 62)), d);
+    split_digits(llrintl(ldexpl(v * (neg ? -c : c), 62)), d);
     unsigned short* t = &tab[(size_t)q * 8];
     for (int s = 0; s < 5; ++s) t[s] = bf16_bits(d[s]);
     t[5] = bf16_bits(d[4] - bf16_float(t[4]));
   }
   const int nrows = form == 0 ? D / 2 + 1 : (nout + 1) / 2;
   const int kp = pad_k(D / 2 + 1);
-  uint4* dtab = nullptr;
   void* mat = nullptr;
-  if (cudaMalloc(&dtab, tab.size() * 2) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
   if (cudaMalloc(&mat, (size_t)2 * kS * nrows * kp * 2) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(dtab);
     return false;
   }
   allocs.push_back(mat);
-  cudaMemcpy(dtab, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice);
-  k_tc_matrix<<<1024, 256>>>(dtab, (__nv_bfloat16*)mat, D, form, nrows, kp);
-  const bool ok = cudaStreamSynchronize(0) == cudaSuccess && cudaGetLastError() == cudaSuccess;
-  cudaFree(dtab);
-  if (!ok) return false;
+  if (cudaMemcpy(scratch, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice) != cudaSuccess) return false;
+  k_tc_matrix<<<1024, 256>>>((const uint4*)scratch, (__nv_bfloat16*)mat, D, form, nrows, kp);
+  if (cudaGetLastError() != cudaSuccess) return false;
   out->D = D;
   out->form = form;
   out->sin_kind = sin_kind;
