@@ -253,27 +253,33 @@ __global__ void __launch_bounds__(kXThreads) axis_pass_lanes_k(const AxisBatchT<
 }
 
 constexpr int kYThreads = 64;
-constexpr int kYR = 8;  // outputs per thread
+constexpr int kYR = 8;  // outputs per thread, or 4 or 2
 
 // y pass: one thread = one line (consecutive lines are contiguous in memory)
-// and kYR lane outputs; twiddles are warp-uniform.  The two symmetries of
+// and R lane outputs; twiddles are warp-uniform.  The two symmetries of
 // the x pass halve the FP64 work of REDFT00 / RODFT00 kinds:
 //   mode 1: lane output k (k <= D/2) keeps even-j and odd-j sums E, O and
 //           writes out[k] and out[D-k]
 //   mode 2: inputs are paired, u = x_j + x_{D-j}, v = x_j - x_{D-j}
 //           (outputs k <= D/2)
-// kYR consecutive twiddles of a y row (rows are 64-byte aligned)
-__device__ __forceinline__ void row8(const double* __restrict__ p, double (&t)[kYR]) {
+// The FP64 pipe bounds it: a warp's multiply-add takes its scheduler 64 cycles, so
+// eight outputs over 72 terms are 18 us for a warp however few there are.  Where
+// that is the longer part (lanes_line_outputs) a thread takes four or two outputs,
+// and the loads of four pairs of terms are in flight (x and y pass of eight fields
+// of 514 x 72 points 79 -> 44 us, of one field 37 -> 22 us).
+// R consecutive twiddles of a y row (rows are 64-byte aligned)
+template <int R>
+__device__ __forceinline__ void twiddle_row(const double* __restrict__ p, double (&t)[R]) {
   const double2* q = reinterpret_cast<const double2*>(p);
 #pragma unroll
-  for (int i = 0; i < kYR / 2; ++i) {
+  for (int i = 0; i < R / 2; ++i) {
     const double2 v = __ldg(q + i);
     t[2 * i] = v.x;
     t[2 * i + 1] = v.y;
   }
 }
 
-template <int NJ>
+template <int NJ, int R>
 __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatchT<NJ> b) {
   pdl_wait();
   int jb = 0;
@@ -285,7 +291,7 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
   const int lb = local - kgrp * nlb;
   const int line = lb * kYThreads + threadIdx.x;
   if (line >= J.nlines) return;
-  const int k0 = kgrp * kYR;
+  const int k0 = kgrp * R;
   const int D = J.D, D4 = 4 * D;
   const double* __restrict__ x = J.in + (long long)line * J.in_sl;
   const long long sk = J.in_sk;
@@ -307,52 +313,53 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
     m += inc;
     if (m >= D4) m -= D4;
   };
-  int m[kYR], inc[kYR];
+  int m[R], inc[R];
   const int a0 = max(J.jlo, 1);
 #pragma unroll
-  for (int r = 0; r < kYR; ++r) {
+  for (int r = 0; r < R; ++r) {
     const int kk = J.ak * (k0 + r) + J.bk;
     inc[r] = mod4d((long long)J.aj * kk, D4);
     m[r] = mod4d((long long)(J.aj * a0 + J.bj) * kk + J.off, D4);
   }
   if (J.mode == 1 && J.ty) {
-    // twiddle rows: row j, columns k0 .. k0 + kYR - 1
+    // twiddle rows: row j, columns k0 .. k0 + R - 1
     const double* __restrict__ T = J.ty + k0;
     const long long ld = J.ldy;
-    double E[kYR], O[kYR], t[kYR];
+    double E[R], O[R], t[R];
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) E[r] = O[r] = 0.0;
+    for (int r = 0; r < R; ++r) E[r] = O[r] = 0.0;
     const int a1 = min(j_end, J.N - 1);
     int j = a0;
     if (j < a1 && (j & 1)) {
       const double v = X(j);
-      row8(T + j * ld, t);
+      twiddle_row<R>(T + j * ld, t);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) O[r] = fma(v, t[r], O[r]);
+      for (int r = 0; r < R; ++r) O[r] = fma(v, t[r], O[r]);
       ++j;
     }
+#pragma unroll(R < kYR ? 4 : 1)
     for (; j + 1 < a1; j += 2) {
       const double v0 = X(j), v1 = X(j + 1);
-      double t1[kYR];
-      row8(T + j * ld, t);
-      row8(T + (j + 1) * ld, t1);
+      double t1[R];
+      twiddle_row<R>(T + j * ld, t);
+      twiddle_row<R>(T + (j + 1) * ld, t1);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         E[r] = fma(v0, t[r], E[r]);
         O[r] = fma(v1, t1[r], O[r]);
       }
     }
     if (j < a1) {
       const double v = X(j);
-      row8(T + j * ld, t);
+      twiddle_row<R>(T + j * ld, t);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) E[r] = fma(v, t[r], E[r]);
+      for (int r = 0; r < R; ++r) E[r] = fma(v, t[r], E[r]);
     }
-    double t0[kYR], tD[kYR];
-    row8(T, t0);
-    row8(T + D * ld, tD);
+    double t0[R], tD[R];
+    twiddle_row<R>(T, t0);
+    twiddle_row<R>(T + D * ld, tD);
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int k = k0 + r;
       if (k >= J.nlane) break;
       double e = J.wm * E[r], o = J.wm * O[r];
@@ -368,25 +375,26 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
   } else if (J.mode == 2 && J.ty) {
     const double* __restrict__ T = J.ty + k0;
     const long long ld = J.ldy;
-    double acc[kYR], t[kYR];
+    double acc[R], t[R];
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) acc[r] = 0.0;
+    for (int r = 0; r < R; ++r) acc[r] = 0.0;
     const int pe = (D + 1) / 2;  // interior pairs j < D - j
+#pragma unroll(R < kYR ? 4 : 1)
     for (int j = 1; j < pe; ++j) {
       const double xa = X(j), xb = X(D - j);
       const double u = xa + xb, v = xa - xb;
-      row8(T + j * ld, t);
+      twiddle_row<R>(T + j * ld, t);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         const bool use_v = (((k0 + r) & 1) == 0) != !is_sin;
         acc[r] = fma(use_v ? v : u, t[r], acc[r]);
       }
     }
-    double t0[kYR], tm[kYR];
-    row8(T, t0);
-    row8(T + (D / 2) * ld, tm);
+    double t0[R], tm[R];
+    twiddle_row<R>(T, t0);
+    twiddle_row<R>(T + (D / 2) * ld, tm);
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int k = k0 + r;
       if (k >= J.nlane) break;
       double tt = J.wm * acc[r];
@@ -401,15 +409,15 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
       put(k, tt);
     }
   } else if (J.mode == 1) {
-    double E[kYR], O[kYR];
+    double E[R], O[R];
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) E[r] = O[r] = 0.0;
+    for (int r = 0; r < R; ++r) E[r] = O[r] = 0.0;
     const int a1 = min(j_end, J.N - 1);
     int j = a0;
     if (j < a1 && (j & 1)) {
       const double v = X(j);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         O[r] = fma(v, twiddle(J.q, D, m[r]), O[r]);
         step(m[r], inc[r]);
       }
@@ -418,7 +426,7 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
     for (; j + 1 < a1; j += 2) {
       const double v0 = X(j), v1 = X(j + 1);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         E[r] = fma(v0, twiddle(J.q, D, m[r]), E[r]);
         step(m[r], inc[r]);
         O[r] = fma(v1, twiddle(J.q, D, m[r]), O[r]);
@@ -428,10 +436,10 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
     if (j < a1) {
       const double v = X(j);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) E[r] = fma(v, twiddle(J.q, D, m[r]), E[r]);
+      for (int r = 0; r < R; ++r) E[r] = fma(v, twiddle(J.q, D, m[r]), E[r]);
     }
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int k = k0 + r;
       if (k >= J.nlane) break;
       double e = J.wm * E[r], o = J.wm * O[r];
@@ -446,23 +454,23 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
       if (D - k != k) put(D - k, is_sin ? o - e : e - o);
     }
   } else if (J.mode == 2) {
-    double acc[kYR];
+    double acc[R];
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) acc[r] = 0.0;
+    for (int r = 0; r < R; ++r) acc[r] = 0.0;
     // cos: even k pairs with u; sin: even k pairs with v
     const int pe = (D + 1) / 2;  // interior pairs j < D - j
     for (int j = 1; j < pe; ++j) {
       const double xa = X(j), xb = X(D - j);
       const double u = xa + xb, v = xa - xb;
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         const bool use_v = (((k0 + r) & 1) == 0) != !is_sin;
         acc[r] = fma(use_v ? v : u, twiddle(J.q, D, m[r]), acc[r]);
         step(m[r], inc[r]);
       }
     }
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int k = k0 + r;
       if (k >= J.nlane) break;
       double t = J.wm * acc[r];
@@ -479,20 +487,20 @@ __global__ void __launch_bounds__(kYThreads) axis_pass_lanes_line(const AxisBatc
       put(k, t);
     }
   } else {
-    double acc[kYR];
+    double acc[R];
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) acc[r] = 0.0;
+    for (int r = 0; r < R; ++r) acc[r] = 0.0;
     const int a1 = min(j_end, J.N - 1);
     for (int j = a0; j < a1; ++j) {
       const double v = X(j);
 #pragma unroll
-      for (int r = 0; r < kYR; ++r) {
+      for (int r = 0; r < R; ++r) {
         acc[r] = fma(v, twiddle(J.q, D, m[r]), acc[r]);
         step(m[r], inc[r]);
       }
     }
 #pragma unroll
-    for (int r = 0; r < kYR; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int k = k0 + r;
       if (k >= J.nout) break;
       double t = J.wm * acc[r];
@@ -1958,6 +1966,29 @@ void launch_tensor(AxisBatch& b, const Tables& tb, cudaStream_t st, AxisBatch* n
     for (int i = 0; i < t.njobs; ++i) next->job[from[i]].lmax = t.job[i].cmax;
 }
 
+// Outputs per thread of axis_pass_lanes_line: its time is the FP64 instructions of
+// the longest warp and those of all warps over the schedulers.  Fewer outputs per
+// thread shorten the first and lengthen the second where terms are paired (two
+// additions per pair and thread); eight unless it saves a tenth, as more threads
+// read the lines and the twiddles again.
+int lanes_line_outputs(const AxisBatch& b, int nsm) {
+  auto cost = [&](int r) {
+    double longest = 0.0, all = 0.0;
+    for (int i = 0; i < b.njobs; ++i) {
+      const AxisJob& J = b.job[i];
+      const double terms = J.mode == 2 ? (J.D + 1) / 2 : std::max(std::min(std::min(J.jhi, J.nin), J.N) - J.jlo, 1);
+      const double ops = terms * (r + (J.mode == 2 ? 2 : 0));
+      longest = std::max(longest, ops);
+      all += ops * ((J.nlines + kYThreads - 1) / kYThreads) * (kYThreads / 32) * ((J.nlane + r - 1) / r);
+    }
+    return longest + all / (4.0 * std::max(nsm, 1));
+  };
+  int best = kYR;
+  for (int r = kYR / 2; r >= 2; r /= 2)
+    if (cost(r) < 0.9 * cost(kYR) && cost(r) < cost(best)) best = r;
+  return best;
+}
+
 // y passes: two-level where the length factors well (scratch permitting),
 // direct sums otherwise
 void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
@@ -2043,7 +2074,6 @@ void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
     b = rest;
   }
   if (b.njobs == 0) return;
-  int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
     AxisJob& J = b.job[i];
     const bool c1s1 = (J.aj == 2 && J.bj == 0 && J.ak == 1 && J.bk == 0);
@@ -2059,15 +2089,21 @@ void launch_batch_y(AxisBatch& in, const Tables& tb, cudaStream_t st) {
       const int nin = std::min(std::min(J.jhi, J.nin), J.N) - J.jlo;
       g_xform_fmas += (double)J.nlines * J.nlane * (J.mode == 2 ? (J.D + 1) / 2 : std::max(nin, 1));
     }
+  }
+  const int R = lanes_line_outputs(b, tb.nsm);
+  int total = 0;
+  for (int i = 0; i < b.njobs; ++i) {
     b.start[i] = total;
-    const int nlb = (J.nlines + kYThreads - 1) / kYThreads;
-    total += nlb * ((J.nlane + kYR - 1) / kYR);
+    total += (b.job[i].nlines + kYThreads - 1) / kYThreads * ((b.job[i].nlane + R - 1) / R);
   }
   b.start[b.njobs] = total;
   if (total > 0)
     with_capacity(b.njobs, [&](auto c) {
       constexpr int NJ = decltype(c)::value;
-      launch_pdl(axis_pass_lanes_line<NJ>, dim3(total), dim3(kYThreads), 0, st, shrink<NJ>(b));
+      launch_pdl(R == 2   ? axis_pass_lanes_line<NJ, 2>
+                 : R == 4 ? axis_pass_lanes_line<NJ, 4>
+                          : axis_pass_lanes_line<NJ, kYR>,
+                 dim3(total), dim3(kYThreads), 0, st, shrink<NJ>(b));
     });
 }
 
