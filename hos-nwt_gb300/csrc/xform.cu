@@ -1582,14 +1582,16 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
       with_capacity(nj, [&](auto c) {
         constexpr int NJ = decltype(c)::value;
         allow_smem(two_level_pass1<NJ>);
-        allow_smem(two_level_pass2<NJ, 8>);
         allow_smem(two_level_pass2<NJ, 16>);
         allow_smem(two_level_pass2<NJ, 32>);
       });
   });
-  // pass 1: as many parts per sum as keep the launch within two CTAs per SM
-  // (each part costs its share of the final sums: 16 of them make the FP64
-  // work of one line 1.4 times that of four)
+  // pass 1: as many parts per sum as keep the launch within half of the SMs.
+  // The right-hand side runs three branches at a time, and the CTAs of their
+  // next passes wait on the SMs too: with launches of two CTAs per SM and eight
+  // outputs per CTA of pass 2 a step of 257 modes took 0.49 to 0.75 ms from
+  // one to the next, with these it takes 0.48 to 0.50, one of 1025 modes
+  // 0.91 ms for 1.07 (a third or a quarter of the SMs: 0.93 to 0.98).
   auto ctas1 = [&](int P) {
     long long n = 0;
     for (int i = 0; i < b.njobs; ++i) {
@@ -1600,7 +1602,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     return n;
   };
   int P = 16;
-  while (P > 2 && ctas1(P) > 2LL * std::max(nsm, 1)) P /= 2;
+  while (P > 2 && 2 * ctas1(P) > std::max(nsm, 1)) P /= 2;
   size_t smem1 = 0, smem2 = 0;
   int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
@@ -1641,14 +1643,13 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     });
     return;
   }
-  // pass 2: fewer outputs per CTA until the launch covers the SMs
+  // pass 2: 16 outputs per CTA where 32 do not cover the SMs
   auto ctas2 = [&](int KO) {
     long long n = 0;
     for (int i = 0; i < b.njobs; ++i) n += (long long)b.job[i].nlines * ((p2_lanes(b.job[i]) + KO - 1) / KO);
     return n;
   };
-  int KO = 32;
-  while (KO > 8 && ctas2(KO) < std::max(nsm, 1)) KO /= 2;
+  const int KO = ctas2(32) < std::max(nsm, 1) ? 16 : 32;
   total = 0;
   for (int i = 0; i < b.njobs; ++i) {
     b.start[i] = total;
@@ -1659,8 +1660,7 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   if (total > 0)
     with_capacity(b.njobs, [&](auto c) {
       constexpr int NJ = decltype(c)::value;
-      if (KO == 8) launch_pdl(two_level_pass2<NJ, 8>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
-      else if (KO == 16) launch_pdl(two_level_pass2<NJ, 16>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
+      if (KO == 16) launch_pdl(two_level_pass2<NJ, 16>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
       else launch_pdl(two_level_pass2<NJ, 32>, dim3(total), dim3(kP2Threads), smem2, st, shrink<NJ>(b));
     });
 }
