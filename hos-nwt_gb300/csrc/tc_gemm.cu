@@ -15,15 +15,13 @@
 //     last commit signals the epilogue;
 //   - all eight warps: tcgen05.ld of their 32 accumulator lanes (two warps per
 //     32 lanes, half of the columns each), bias and activation, stores.
-// A product of few tiles and many terms (a truncated transform of 2052 points, the
-// weight gradients of small batches) is cut along K (split_count): every slice
-// writes its FP32 sums to the caller's workspace and k_tc_reduce adds them in a
-// fixed order.
-// Measured (with views read in place, before -> now, a call alone): 65664 x 32 over
-// 32 modes of a grid 42 -> 37 us, the larger drawn contractions 105 -> 68 us;
-// kernel only: 32 x 32 over 65664 terms 299 -> 150 us, over 6144 33 -> 21 us,
-// 8192^3 1.29 -> 1.19 ms.  A single tile over many terms is bound by the latency of
-// the ring (about 280 cycles for a stage of 64 terms), a narrow product by memory.
+// Measured (with views read in place, before -> now, a call alone): 32896 x 64 over
+// 2056 terms 42 -> 37 us, 10919 x 255 over 64 terms 43 -> 23 us; kernel only: 32 x 32
+// over 65664 terms 299 -> 150 us, over 6144 33 -> 21 us, 8192^3 1.29 -> 1.19 ms.
+// A single tile over many terms is bound by the latency of the ring (about 280
+// cycles for a stage of 64 terms), a narrow product by memory.  Cutting K over
+// idle SMs does not pay below 6144 terms: a stage takes 0.14 us, the second
+// launch and the workspace 9 us.
 // Every wait on an mbarrier is bounded: on timeout the CTA records an error
 // code in a device flag, skips its remaining work, frees its tensor memory
 // and returns.
@@ -188,10 +186,7 @@ struct GemmArgs {
   const float* bias;   // N entries or null
   int act;             // 0 none, 1 GELU
   const float* Dadd;   // optional FP32 M x N (ldd) added before the activation
-  int kb_per;          // stages per slice of K
   int rows_a, rows_b;  // rows of a K-major box: the tile's, but no more than the matrix has
-                       // also where it lies outside the matrix
-  float* part;         // slices > 1: FP32 sums [slice][M][N], else null
   unsigned* err;       // error flag (1: a wait timed out; 2: the wait for the
                        // MMAs to finish timed out too, so the CTA exited
                        // without freeing its tensor memory: treat the
@@ -206,26 +201,6 @@ __device__ __forceinline__ void store_out(const GemmArgs& g, int row, int col, f
     ((__nv_bfloat16*)g.D)[o] = __float2bfloat16(x);
   else
     ((float*)g.D)[o] = x;
-}
-
-// D from the slices' sums: 32 outputs per block, 8 warps over the slices
-__global__ void __launch_bounds__(256) k_tc_reduce(GemmArgs g, int slices) {
-  __shared__ float red[8][32];
-  const long long n = (long long)g.M * g.N;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long i = blockIdx.x * 32LL + lane;
-  float x = 0.0f;
-  if (i < n)
-#pragma unroll 4
-    for (int s = warp; s < slices; s += 8) x += __ldcg(g.part + s * n + i);
-  red[warp][lane] = x;
-  __syncthreads();
-  if (warp == 0 && i < n) {
-    const float y = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) +
-                    ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
-    const int row = (int)(i / g.N), col = (int)(i - (long long)row * g.N);
-    store_out(g, row, col, y + (g.bias ? g.bias[col] : 0.0f));
-  }
 }
 
 template <int BN, bool TA, bool TB, int kStages>
@@ -245,8 +220,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ int n_issued, n_consumed;  // stages loaded by TMA / read by the MMAs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-  const int kb0 = blockIdx.z * g.kb_per;
-  const int nk = min((g.K + kBK - 1) / kBK - kb0, g.kb_per);
+  const int nk = (g.K + kBK - 1) / kBK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -284,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         break;
       }
       mbar_expect_tx(&full_bar[s], bytes_a + bytes_b, elected);
-      const int k0 = (kb0 + kb) * kBK;
+      const int k0 = kb * kBK;
       if constexpr (TA) {
         for (int q = 0; q < blk_a; ++q)
           tma_load_2d(sA + s * kABytes + q * (kBK * 128), &mapA, m0 + 64 * q, k0, &full_bar[s], elected);
@@ -362,15 +336,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 4
       for (int r = half; r < 32; r += 2) {
         const int row = m0 + quad * 32 + r;
-        if (row < g.M && col < g.N) {
-          float x = tile[r * 17 + cl];
-          if (g.part) {
-            g.part[((long long)blockIdx.z * g.M + row) * g.N + col] = x;
-          } else {
-            x += bcol;
-            store_out(g, row, col, x);
-          }
-        }
+        if (row < g.M && col < g.N) store_out(g, row, col, tile[r * 17 + cl] + bcol);
       }
       __syncwarp();
     }
@@ -437,43 +403,25 @@ cudaError_t launch_ring(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm
 }
 
 template <int BN, bool TA, bool TB>
-cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, int slices, cudaStream_t st) {
-  const dim3 grid((g.M + kBM - 1) / kBM, (g.N + BN - 1) / BN, slices);
-  if ((long long)grid.x * grid.y * grid.z <= sm_count())
+cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, cudaStream_t st) {
+  const dim3 grid((g.M + kBM - 1) / kBM, (g.N + BN - 1) / BN);
+  if (g.K > kStagesFew * kBK && (long long)grid.x * grid.y <= sm_count())
     return launch_ring<BN, TA, TB, kStagesDeep<BN>>(ma, mb, g, grid, st);
   return launch_ring<BN, TA, TB, kStagesFew>(ma, mb, g, grid, st);
 }
 
 int tile_cols(int N) { return N <= 32 ? 32 : (N <= 64 ? 64 : 128); }
 
-// Slices of K: where the tiles leave most SMs idle and a slice keeps four
-// stages (a slice costs its 4 bytes per output twice, and the reduction a
-// launch of 3 us; below 16 stages the product itself takes less).  Sums longer than
-// 6144 terms stay whole: their FP32 accumulation is off by up to 8e-5 of the
-// result, and a call keeps the value that one accumulator gives.
-int split_count(int M, int N, int K) {
-  const int nsm = sm_count(), bn = tile_cols(N);
-  const long long tiles = ((long long)M + kBM - 1) / kBM * ((N + bn - 1) / bn);
-  const int kb = (K + kBK - 1) / kBK;
-  if (kb < 16 || K > 6144 || 2 * tiles > nsm) return 1;
-  const int want = (int)std::min<long long>(nsm / tiles, kb / 4);
-  if (want < 2) return 1;
-  const int per = (kb + want - 1) / want;
-  return (kb + per - 1) / per;
-}
-
 }  // namespace
 
 // D = act(A B^T + bias [+ Dadd]); see the file comment.  A: M x K with row
 // stride lda, or its transpose K x M (ta); B: N x K, or K x N (tb), both BF16;
 // lda and ldb multiples of 8, K a multiple of 8 where an operand has it
-// contiguous, both base addresses 16-byte aligned (the TMA rules).  work holds
-// split_count(M, N, K) * M * N floats where that count is above one (else, or
-// null, K is not cut).  Returns a cudaError_t value (cudaErrorInvalidValue for
-// shapes the kernel does not take).
+// contiguous, both base addresses 16-byte aligned (the TMA rules).  Returns a
+// cudaError_t value (cudaErrorInvalidValue for shapes the kernel does not take).
 int tc_gemm_bf16(const void* A, long long lda, bool ta, const void* B, long long ldb, bool tb, void* D, long long ldd,
-                 int d_bf16, int M, int N, int K, const float* bias, int act, const float* Dadd, float* work,
-                 unsigned* err, cudaStream_t st) {
+                 int d_bf16, int M, int N, int K, const float* bias, int act, const float* Dadd, unsigned* err,
+                 cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0 || (!(ta && tb) && (K % 8)) || (lda % 8) || (ldb % 8) || ((uintptr_t)A & 15) ||
       ((uintptr_t)B & 15) || !err)
     return (int)cudaErrorInvalidValue;
@@ -485,26 +433,18 @@ int tc_gemm_bf16(const void* A, long long lda, bool ta, const void* B, long long
   if (!(ta ? make_map(&ma, A, K, M, lda, kBK) : make_map(&ma, A, M, K, lda, rows_a)) ||
       !(tb ? make_map(&mb, B, K, N, ldb, kBK) : make_map(&mb, B, N, K, ldb, rows_b)))
     return (int)cudaErrorInvalidValue;
-  const int kb = (K + kBK - 1) / kBK;
-  const int slices = work ? split_count(M, N, K) : 1;
-  GemmArgs g{M, N, K, D, ldd, d_bf16, bias, act, Dadd, (kb + slices - 1) / slices, rows_a, rows_b,
-             slices > 1 ? work : nullptr, err};
+  GemmArgs g{M, N, K, D, ldd, d_bf16, bias, act, Dadd, rows_a, rows_b, err};
   cudaError_t e = cudaSuccess;
   auto go = [&](auto bnc) {
     constexpr int BN = decltype(bnc)::value;
-    if (ta && tb) e = launch_gemm<BN, true, true>(ma, mb, g, slices, st);
-    else if (ta) e = launch_gemm<BN, true, false>(ma, mb, g, slices, st);
-    else if (tb) e = launch_gemm<BN, false, true>(ma, mb, g, slices, st);
-    else e = launch_gemm<BN, false, false>(ma, mb, g, slices, st);
+    if (ta && tb) e = launch_gemm<BN, true, true>(ma, mb, g, st);
+    else if (ta) e = launch_gemm<BN, true, false>(ma, mb, g, st);
+    else if (tb) e = launch_gemm<BN, false, true>(ma, mb, g, st);
+    else e = launch_gemm<BN, false, false>(ma, mb, g, st);
   };
   if (bn == 32) go(std::integral_constant<int, 32>());
   else if (bn == 64) go(std::integral_constant<int, 64>());
   else go(std::integral_constant<int, 128>());
-  if (e == cudaSuccess && slices > 1) {
-    const long long n = (long long)M * N;
-    k_tc_reduce<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(g, slices);
-    e = cudaGetLastError();
-  }
   return (int)e;
 }
 
@@ -517,21 +457,13 @@ static int gemm_status(int e) {
 extern "C" int hosnwt_tc_gemm_bf16(const void* A, long long lda, const void* B, long long ldb, void* D,
                                    long long ldd, int d_bf16, int M, int N, int K, const float* bias, int act,
                                    const float* Dadd, unsigned* err, void* stream) {
-  return gemm_status(hos::tc_gemm_bf16(A, lda, false, B, ldb, false, D, ldd, d_bf16, M, N, K, bias, act, Dadd, nullptr,
-                                       err, (cudaStream_t)stream));
+  return gemm_status(hos::tc_gemm_bf16(A, lda, false, B, ldb, false, D, ldd, d_bf16, M, N, K, bias, act, Dadd, err,
+                                       (cudaStream_t)stream));
 }
 
-extern "C" long long hosnwt_tc_gemm_workspace(int M, int N, int K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int s = hos::split_count(M, N, K);
-  return s > 1 ? 4LL * s * M * N : 0;
-}
-
-extern "C" int hosnwt_tc_gemm_bf16_ex(const void* A, long long lda, int ta, const void* B, long long ldb, int tb,
-                                      void* D, long long ldd, int d_bf16, int M, int N, int K, const float* bias,
-                                      int act, const float* Dadd, void* work, long long work_bytes, unsigned* err,
-                                      void* stream) {
-  if (work && work_bytes < hosnwt_tc_gemm_workspace(M, N, K)) return HOSNWT_ERR_ARG;
-  return gemm_status(hos::tc_gemm_bf16(A, lda, ta != 0, B, ldb, tb != 0, D, ldd, d_bf16, M, N, K, bias, act, Dadd,
-                                       (float*)work, err, (cudaStream_t)stream));
+extern "C" int hosnwt_tc_gemm_bf16_views(const void* A, long long lda, int ta, const void* B, long long ldb, int tb,
+                                         void* D, long long ldd, int d_bf16, int M, int N, int K, const float* bias,
+                                         int act, const float* Dadd, unsigned* err, void* stream) {
+  return gemm_status(hos::tc_gemm_bf16(A, lda, ta != 0, B, ldb, tb != 0, D, ldd, d_bf16, M, N, K, bias, act, Dadd, err,
+                                       (cudaStream_t)stream));
 }

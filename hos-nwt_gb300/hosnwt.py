@@ -107,10 +107,8 @@ def load_library(path=LIB_PATH):
     ll = ctypes.c_longlong
     ci = ctypes.c_int
     lib.hosnwt_tc_gemm_bf16.argtypes = [vp8, ll, vp8, ll, vp8, ll, ci, ci, ci, ci, vp8, ci, vp8, vp8, vp8]
-    lib.hosnwt_tc_gemm_bf16_ex.argtypes = [vp8, ll, ci, vp8, ll, ci, vp8, ll, ci, ci, ci, ci, vp8, ci, vp8, vp8, ll,
-                                           vp8, vp8]
-    lib.hosnwt_tc_gemm_workspace.argtypes = [ci, ci, ci]
-    lib.hosnwt_tc_gemm_workspace.restype = ll
+    lib.hosnwt_tc_gemm_bf16_views.argtypes = [vp8, ll, ci, vp8, ll, ci, vp8, ll, ci, ci, ci, ci, vp8, ci, vp8,
+                                              vp8, vp8]
     _lib = lib
     return lib
 
@@ -390,33 +388,31 @@ def tc_gemm(A, B, bias=None, act=0, Dadd=None, out=None, out_bf16=False, err=Non
         out = torch.empty((M, N), dtype=torch.bfloat16 if out_bf16 else torch.float32, device=A.device)
     if err is None:
         err = torch.zeros(1, dtype=torch.int32, device=A.device)
-    return tc_gemm_views(A, B, False, False, bias, act, Dadd, out, err, stream)
-
-
-def tc_gemm_views(A, B, ta, tb, bias, act, Dadd, out, err, stream, current=None):
-    """tc_gemm on operands as they lie (hosnwt_tc_gemm_bf16_ex): A is M x K,
-    or K x M with `ta`; B is N x K, or K x N with `tb`; rows contiguous.  A
-    product of few tiles and many terms is cut along K, with a workspace from
-    PyTorch's allocator, if `stream` is the current stream (the allocator
-    orders its memory by that one; `current`, if the caller knows it)."""
-    import torch
-    lib = load_library()
-    M, K = (A.shape[1], A.shape[0]) if ta else A.shape
-    N = B.shape[1] if tb else B.shape[0]
     # the row stride of a one-row matrix is arbitrary in PyTorch (a transposed
     # column reports 1); the kernel never steps over it, so pass the row length
-    lda = A.stride(0) if A.shape[0] > 1 else A.shape[1]
-    ldb = B.stride(0) if B.shape[0] > 1 else B.shape[1]
+    lda = A.stride(0) if M > 1 else K
+    ldb = B.stride(0) if N > 1 else K
     ldd = out.stride(0) if M > 1 else N
-    need = lib.hosnwt_tc_gemm_workspace(M, N, K)
-    if need and stream != (torch.cuda.current_stream(A.device).cuda_stream if current is None else current):
-        need = 0
-    work = torch.empty(need // 4, dtype=torch.float32, device=A.device) if need else None
-    rc = lib.hosnwt_tc_gemm_bf16_ex(
-        A.data_ptr(), lda, int(ta), B.data_ptr(), ldb, int(tb), out.data_ptr(), ldd,
+    rc = load_library().hosnwt_tc_gemm_bf16(
+        A.data_ptr(), lda, B.data_ptr(), ldb, out.data_ptr(), ldd,
         1 if out.dtype == torch.bfloat16 else 0, M, N, K, bias.data_ptr() if bias is not None else None,
-        int(act), Dadd.data_ptr() if Dadd is not None else None, work.data_ptr() if need else None, need,
-        err.data_ptr(), stream)
+        int(act), Dadd.data_ptr() if Dadd is not None else None, err.data_ptr(), stream)
     if rc != HOSNWT_OK:
         raise HosError(f"hosnwt_tc_gemm_bf16 failed ({ERRORS.get(rc, rc)})")
+    return out
+
+
+def tc_gemm_views(A, B, ta, tb, out, err, stream):
+    """D = A B^T (FP32) on operands as they lie (hosnwt_tc_gemm_bf16_views): A
+    is M x K, or K x M with `ta`; B is N x K, or K x N with `tb`; rows
+    contiguous."""
+    M, K = (A.shape[1], A.shape[0]) if ta else A.shape
+    N = B.shape[1] if tb else B.shape[0]
+    lda = A.stride(0) if A.shape[0] > 1 else A.shape[1]
+    ldb = B.stride(0) if B.shape[0] > 1 else B.shape[1]
+    rc = load_library().hosnwt_tc_gemm_bf16_views(
+        A.data_ptr(), lda, int(ta), B.data_ptr(), ldb, int(tb), out.data_ptr(), out.stride(0) if M > 1 else N, 0, M, N, K,
+        None, 0, None, err.data_ptr(), stream)
+    if rc != HOSNWT_OK:
+        raise HosError(f"hosnwt_tc_gemm_bf16_views failed ({ERRORS.get(rc, rc)})")
     return out

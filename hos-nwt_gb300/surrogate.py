@@ -90,8 +90,7 @@ def gemm_bf16(A, B):
         a, ta = _operand(A, False)
         b, tb = _operand(B, False)
     out = torch.empty((M, N), dtype=torch.float32, device=A.device)
-    st = torch.cuda.current_stream(A.device).cuda_stream
-    return hosnwt.tc_gemm_views(a, b, ta, tb, None, 0, None, out, _err_flag(A.device), st, st)
+    return hosnwt.tc_gemm_views(a, b, ta, tb, out, _err_flag(A.device), torch.cuda.current_stream(A.device).cuda_stream)
 
 
 def check_kernel_flags():

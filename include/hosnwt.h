@@ -230,16 +230,12 @@ int hosnwt_tc_gemm_bf16(const void* A, long long lda, const void* B, long long l
                         int d_bf16, int M, int N, int K, const float* bias, int act, const float* Dadd,
                         unsigned* err, void* stream);
 
-/* The same contraction with operands as they lie and a workspace.  ta: A is
- * given as its transpose, K x M with row stride lda; tb: B as K x N with row
- * stride ldb (K must be a multiple of 8 unless both are).  work (device, may be
- * null) of at least hosnwt_tc_gemm_workspace(M, N, K) bytes lets a product of
- * few tiles and 1024 to 6144 terms be cut along K; its slices are added in a
- * fixed order.  hosnwt_tc_gemm_workspace gives 0 where K is not cut. */
-long long hosnwt_tc_gemm_workspace(int M, int N, int K);
-int hosnwt_tc_gemm_bf16_ex(const void* A, long long lda, int ta, const void* B, long long ldb, int tb, void* D,
-                           long long ldd, int d_bf16, int M, int N, int K, const float* bias, int act,
-                           const float* Dadd, void* work, long long work_bytes, unsigned* err, void* stream);
+/* The same contraction with operands as they lie.  ta: A is given as its
+ * transpose, K x M with row stride lda; tb: B as K x N with row stride ldb (K
+ * must be a multiple of 8 unless both are). */
+int hosnwt_tc_gemm_bf16_views(const void* A, long long lda, int ta, const void* B, long long ldb, int tb, void* D,
+                              long long ldd, int d_bf16, int M, int N, int K, const float* bias, int act,
+                              const float* Dadd, unsigned* err, void* stream);
 
 #ifdef __cplusplus
 }
