@@ -4,8 +4,9 @@ M = 7, p1 = p2 = 7, dealiased grid 4100 x 2052; 50 m x 30 m x 5 m, snake
 flap, JONSWAP Hs = 0.15 m, Tp = 1.3 s, gamma = 5, cos^2s spreading s = 15;
 synthetic seeded phases and directions), the largest benchmark
 configuration, run on the plain path (FP64 state, right-hand side and RK
-stages; the FFT passes' complex DFT in double-float, HOSNWT_FFT_DF=0 for
-FP64).
+stages; the large transform passes as exact digit products on the tensor
+cores, the FFT passes' complex DFT in double-float; HOSNWT_FFT_DF=0 for FP64
+passes).
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl cuda|reference]
                   [--workload steep_3d|directional_3d|irregular_2d|regular_2d|...]
@@ -507,13 +508,15 @@ def run_cuda(args, w):
                              "ms_per_launch": ms,
                              "timing": "the transform's launches, 20 replays in one CUDA graph, CUDA events on "
                                        "the library's stream",
-                             "note": ("not HBM bound: the passes' DFT runs in double-float on the FP32 pipe "
-                                      "(bound by instruction issue); fp64_step gives the step's transform work "
-                                      "in FP64 instructions against the FP64 peak" if df else
+                             "note": ("not HBM bound: the large passes run as digit products at the tensor "
+                                      "cores' BF16 rate, the others in double-float on the FP32 pipe; fp64_step "
+                                      "gives the step's transform work in FP64 instructions against the FP64 "
+                                      "peak" if df else
                                       "FP64-pipe bound, not HBM bound: GB300 runs FP64 at about 1.2 TFLOP/s; "
                                       "fp64_step gives the step's transform FMAs against the FP64 peak")},
-                "arithmetic": ("FP64 state, right-hand side and RK stages; the FFT passes' complex DFT in "
-                               "double-float (pairs of FP32, 48-bit significand)" if df else
+                "arithmetic": ("FP64 state, right-hand side and RK stages; large transform passes as exact "
+                               "sums of BF16 digit products in 64-bit fixed point, the FFT passes' complex DFT "
+                               "in double-float (pairs of FP32, 48-bit significand)" if df else
                                "FP64 throughout" + (" (HOSNWT_FFT_DF=0)" if n2 > 1 else
                                                     " (a 2-D tank: FP64 sum passes)")),
                 }
