@@ -510,8 +510,8 @@ def run_cuda(args, w):
                                        "the library's stream",
                              "note": ("not HBM bound: the large passes run as digit products at the tensor "
                                       "cores' BF16 rate, the others in double-float on the FP32 pipe; fp64_step "
-                                      "gives the step's transform work in FP64 instructions against the FP64 "
-                                      "peak" if df else
+                                      "gives the multiply-adds of the passes as they run (matrix products "
+                                      "included) against the FP64 peak" if df else
                                       "FP64-pipe bound, not HBM bound: GB300 runs FP64 at about 1.2 TFLOP/s; "
                                       "fp64_step gives the step's transform FMAs against the FP64 peak")},
                 "arithmetic": ("FP64 state, right-hand side and RK stages; large transform passes as exact "

@@ -1,6 +1,6 @@
 // FFT-based transform passes of the HOS-NWT hot path on sm_103a.
 //
-// Replaces, for the axis passes over many lines (every pass of a 3-D tank),
+// Replaces, for the axis passes over many lines (the passes of a 3-D tank that tcx.cu leaves),
 // the FFTW r2r plans of fourier_FFTW.f90:130-167 (REDFT00 for the cos
 // transforms, RODFT00 on the interior for the sin transforms; S2F/F2S
 // normalisation fourier_FFTW.f90:175-229 applied as the pass's input weights
