@@ -87,8 +87,10 @@ def gemm_bf16(A, B):
     b, tb = _operand(B, K <= _LONG_K)
     if ta != tb and K % 8:
         # the padded row of one operand would meet the K rows of the other
-        a, ta = _operand(A, False)
-        b, tb = _operand(B, False)
+        if ta:
+            a, ta = _operand(A, False)
+        else:
+            b, tb = _operand(B, False)
     out = torch.empty((M, N), dtype=torch.float32, device=A.device)
     return hosnwt.tc_gemm_views(a, b, ta, tb, out, _err_flag(A.device), torch.cuda.current_stream(A.device).cuda_stream)
 
