@@ -563,7 +563,10 @@ template <typename T>
 static T* dalloc(Ctx& c, size_t n) {
   void* p = nullptr;
   if (n == 0) n = 1;
-  if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return nullptr;
+  if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) {
+    c.alloc_failed = true;  // the error itself may be read by another call
+    return nullptr;
+  }
   cudaMemset(p, 0, n * sizeof(T));
   c.allocs.push_back(p);
   return (T*)p;
@@ -865,6 +868,9 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
       if (build_fft_plan(D, c.allocs, &f)) c.tb.fft[c.tb.nfft++] = f;
     }
   }
+  // nothing is launched with an array that was refused; the matrices below may
+  // be, and what they find pending would be taken for their own
+  if (c.alloc_failed || cudaPeekAtLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "device allocation failed");
   // matrices of the tensor-core passes: F2S in cos and sin and S2F in cos
   // (what the right-hand side transforms), the S2F of the dealiased grid
   // also truncated to the free-surface modes
@@ -897,8 +903,6 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
     t->nfft = c.tb.nfft;
     for (int i = 0; i < c.tb.nfft; ++i) t->fft[i] = c.tb.fft[i];
   }
-  for (void* p : c.allocs)
-    if (!p) return fail(c, HOSNWT_ERR_CUDA, "device allocation failed");
   if (cudaGetLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "upload failed");
   return HOSNWT_OK;
 }
@@ -970,9 +974,7 @@ int alloc_device(Ctx& c) {
   if (cudaMallocHost((void**)&d.host_io, (2 * nN + (S - (size_t)c.L.off[S_AADD1]) + 1) * sizeof(double)) !=
       cudaSuccess)
     return 1;
-  for (void* p : c.allocs)
-    if (!p) return 1;
-  return 0;
+  return c.alloc_failed ? 1 : 0;
 }
 
 void free_device(Ctx& c) {

@@ -167,6 +167,7 @@ struct Ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int nparts = 0;
   std::vector<void*> allocs;
+  bool alloc_failed = false;      // a device array was refused
 };
 
 // host setup (host.cpp)

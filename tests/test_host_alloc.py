@@ -1,0 +1,46 @@
+"""A device allocation that is refused while a tank is created, each one in
+turn: hosnwt_create reports it and launches nothing afterwards.  What a tank can
+do without (the matrices of the tensor-core passes, the layout tuner's scratch
+outputs) may be refused and the tank still comes up, on the other passes."""
+import pytest
+
+from host_lib import link, run
+
+
+@pytest.fixture(scope="module")
+def host_lib():
+    return link()
+
+
+SCRIPT = r"""
+size = SIZE
+lib.host_cudart_reset()
+t = tank(*size)
+n = lib.host_cudart_mallocs()
+t.close()
+base = lib.host_cudart_bytes()
+came_up, launched, leaked = [], [], []
+for k in range(1, n + 1):
+    lib.host_cudart_reset()
+    lib.host_cudart_refuse(k)
+    try:
+        t = tank(*size)
+        came_up.append(k)
+        t.close()
+    except hosnwt.HosError as e:
+        if lib.host_cudart_launches_after_refusal():
+            launched.append(k)
+    if lib.host_cudart_bytes() != base:
+        leaked.append(k)
+print(json.dumps({"n": n, "came_up": came_up, "launched": launched, "leaked": leaked}))
+"""
+
+
+@pytest.mark.parametrize("size,optional", [((65, 33, 9, 3, 3, 3), 15), ((129, 65, 9, 4, 3, 3, 2), 15), ((65, 1, 9, 3, 3, 1, 2), 0)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else None)
+def test_refused_allocation(host_lib, size, optional):
+    out = run(host_lib, SCRIPT.replace("SIZE", repr(size)), {"HOSNWT_FFT": "2"})
+    print(out)
+    assert out["launched"] == [] and out["leaked"] == []
+    # the optional allocations are the last ones of the creation
+    assert len(out["came_up"]) <= optional and all(k > out["n"] - optional for k in out["came_up"]), out
