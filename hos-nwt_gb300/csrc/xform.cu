@@ -1543,9 +1543,10 @@ void with_capacity(int njobs, F&& f) {
   else if (njobs <= 8) f(std::integral_constant<int, 8>{});
   else f(std::integral_constant<int, kMaxJobs>{});
 }
+constexpr size_t kSmemCap = 200 * 1024;  // dynamic shared memory of a pass
 template <typename K>
 void allow_smem(K kern) {
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
 }
 
 int p1_terms(const AxisJob& J) { return (std::min(J.jhi, J.nin) + J.B - 1) / J.B; }
@@ -1618,10 +1619,16 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
       constexpr int NJ = decltype(c)::value;
       launch_pdl(two_level_pass1<NJ>, dim3(total), dim3(kP1Threads), smem1, st, shrink<NJ>(b), P);
     });
-  // pass 2 with many lines per job: line groups share their staged twiddles
+  // pass 2 with many lines per job: line groups share their staged twiddles; and
+  // with any length whose whole table is over the shared memory (D > 25599), as
+  // these hold B x 32 of them (128 KB at most)
   int minl = 1 << 30;
-  for (int i = 0; i < b.njobs; ++i) minl = std::min(minl, b.job[i].nlines);
-  if (minl >= 16) {
+  size_t table = 0;
+  for (int i = 0; i < b.njobs; ++i) {
+    minl = std::min(minl, b.job[i].nlines);
+    table = std::max(table, pass2_smem(b.job[i]));
+  }
+  if (minl >= 16 || table > kSmemCap) {
     static PerDeviceOnce attr_l;
     attr_l.run([&] {
       for (int nj : {1, 2, 4, 8, kMaxJobs})
@@ -1697,7 +1704,7 @@ bool launch_two_level_fused(AxisBatch& b, int nsm, bool early, cudaStream_t st) 
   const int nsplit = (int)std::max<long long>(1, std::min<long long>(4, std::max(nsm, 1) / units));
   size_t smem = 0;
   for (int i = 0; i < b.njobs; ++i) smem = std::max(smem, fused_smem(b.job[i], nsplit));
-  if (smem > 200 * 1024) return false;
+  if (smem > kSmemCap) return false;
   static PerDeviceOnce attr_set;
   attr_set.run([&] {
     for (int nj : {1, 2, 4, 8, kMaxJobs})
