@@ -1045,6 +1045,11 @@ static int build_step_graph(Ctx& c) {
     fft_tune_record(false);
     c.fmas_per_step = g_xform_fmas - f0;
     if (cudaStreamEndCapture(c.st, &g) != cudaSuccess) return cuda_check(c, "end capture");
+    // a launch that was refused is not in the graph: the step would leave it out
+    if (const int rc = cuda_check(c, "step capture")) {
+      cudaGraphDestroy(g);
+      return rc;
+    }
     if (!record) break;
     const int tuned = fft_tune_run(c.st);
     if (tuned < 0) {
@@ -1339,12 +1344,14 @@ static bool try_build_loop(Ctx& c, bool pdl) {
         cudaSuccess)
       break;
     g_launch_no_pdl = !pdl;
+    const cudaError_t before = cudaPeekAtLastError();
     const double f0 = g_xform_fmas;
     enqueue_ctl_step(c, c.ctl_dev, cp, c.st);
     g_xform_fmas = f0;
     g_launch_no_pdl = false;
     cudaGraph_t captured = nullptr;
     if (cudaStreamEndCapture(c.st, &captured) != cudaSuccess) break;
+    if (cudaPeekAtLastError() != before) break;  // a launch was refused
     if (cudaGraphAddMemcpyNode1D(&n_out, g, &n_loop, 1, c.ctl_host, c.ctl_dev, sizeof(StepCtl),
                                  cudaMemcpyDeviceToHost) != cudaSuccess)
       break;

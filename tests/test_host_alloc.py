@@ -44,3 +44,28 @@ def test_refused_allocation(host_lib, size, optional):
     assert out["launched"] == [] and out["leaked"] == []
     # the optional allocations are the last ones of the creation
     assert len(out["came_up"]) <= optional and all(k > out["n"] - optional for k in out["came_up"]), out
+
+
+LAUNCH_SCRIPT = r"""
+out = []
+for kern in KERNELS:
+    lib.host_cudart_reset()
+    lib.host_cudart_fail_launch(kern.encode())
+    try:
+        t = tank(*SIZE, icase=1)
+        out.append([kern, "came up"])
+        t.close()
+    except hosnwt.HosError as e:
+        out.append([kern, str(e)])
+print(json.dumps(out))
+"""
+
+
+@pytest.mark.parametrize("size", [(65, 1, 9, 3, 3, 1), (65, 33, 9, 3, 3, 3)], ids=lambda v: "x".join(map(str, v)))
+def test_refused_launch(host_lib, size):
+    """A kernel of the step that cannot be launched while the step is captured:
+    hosnwt_create says so (icase 1 launches none of them before)."""
+    kernels = ["k_rk_err", "k_assemble", "k_rk_out"] + (["two_level"] if size[1] == 1 else ["k_fft_pass"])
+    out = run(host_lib, LAUNCH_SCRIPT.replace("SIZE", repr(size)).replace("KERNELS", repr(kernels)))
+    for kern, msg in out:
+        assert "step capture" in msg, (kern, msg)
