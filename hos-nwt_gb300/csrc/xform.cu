@@ -754,8 +754,10 @@ __host__ __device__ inline P1Shape p1_shape(int A, int B, int P) {
 // sin(pi j1 k' / A), so the same four sums give C, S at k' and at A - k' and
 // half of the k' are computed.  Threads own (k', j2, part) with k' fastest:
 // inputs are broadcast, twiddles gathered from the 2 A pairs cos, sin(pi m / A).  The inputs
-// enter with the interior weight 1; pass 2 multiplies the outputs by it.
-template <int NJ>
+// enter with the interior weight 1; pass 2 multiplies the outputs by it.  STAGED:
+// the pairs lie in shared memory; a longer table (A > 5119, so D > 20475 as B is
+// 4 or more) is read from the quarter-wave table in global memory.
+template <int NJ, bool STAGED>
 __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<NJ> b, int P) {
   extern __shared__ double sm1[];
   __shared__ double red[4 * kP1Threads];
@@ -772,15 +774,17 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
   const int j20 = (local % sh.jblocks) * sh.G, line = local / sh.jblocks;
   const int kp0 = kb * sh.nk, nk = min(sh.nk, H + 1 - kp0), G = min(sh.G, B - j20);
   double2* tw = reinterpret_cast<double2*>(sm1);                    // cos, sin(pi m / A), m < 2 A
-  double* xs = sm1 + 4 * (size_t)A;                                 // [j1][j2] inputs, zero outside the sum
+  double* xs = sm1 + (STAGED ? 4 * (size_t)A : 0);                  // [j1][j2] inputs, zero outside the sum
   const double* __restrict__ x = J.in + (long long)line * J.in_sl;
   const double* __restrict__ wr = J.win ? J.win + (long long)line * J.win_sl : nullptr;
   const double* __restrict__ q = J.q;
+  auto pair_of = [&](int t) -> double2 {
+    const int m = 2 * B * t;  // pi t / A = pi m / (2 D), m < 4 D
+    return make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
+  };
   auto stage_twiddles = [&]() {
-    for (int t = threadIdx.x; t < 2 * A; t += kP1Threads) {
-      const int m = 2 * B * t;  // pi t / A = pi m / (2 D), m < 4 D
-      tw[t] = make_double2(twiddle(q, D, m), twiddle(q, D, m >= D ? m - D : m + 3 * D));
-    }
+    if constexpr (STAGED)
+      for (int t = threadIdx.x; t < 2 * A; t += kP1Threads) tw[t] = pair_of(t);
   };
   if (b.early) stage_twiddles();
   const bool half0 = J.w0 != J.wm, halfD = J.wl != J.wm;
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(kP1Threads) two_level_pass1(const AxisBatchT<N
     for (int p = part; p < Kp / 2; p += P) {
       const double v0 = xs[2 * p * G + j2l], v1 = xs[(2 * p + 1) * G + j2l];
       const int m1 = m + kp >= A2 ? m + kp - A2 : m + kp;
-      const double2 t0 = tw[m], t1 = tw[m1];
+      const double2 t0 = STAGED ? tw[m] : pair_of(m), t1 = STAGED ? tw[m1] : pair_of(m1);
       m += inc;
       if (m >= A2) m -= A2;
       ce = fma(v0, t0.x, ce);
@@ -1498,6 +1502,8 @@ int axis_kind(int grid_axis_is_z, int dir, int cs) {
   return cs ? K_S1_F2S : K_C1_F2S;
 }
 
+constexpr size_t kSmemCap = 200 * 1024;  // dynamic shared memory of a pass
+
 // FMAs of a two-level pass pair on one line: pass 1 folds k' about A/2,
 // pass 2 pairs outputs k, D - k when B is even and every output is wanted
 double x_two_level_cost(int A, int B, int D, int nin, int nout) {
@@ -1514,7 +1520,7 @@ void pick_factors(int D, int nin, int nout, int* Aout, int* Bout) {
     if (D % A) continue;
     const int B = D / A;
     if (B < 2 || B > 256) continue;  // pass 2 of many lines stages B x 32 twiddle pairs
-    if (32LL * A + 16LL * (A + 2) > 180 * 1024) continue;  // pass 1's table and inputs
+    if (8LL * (A + 2) > (long long)kSmemCap) continue;  // pass 1's inputs
     const double cost = x_two_level_cost(A, B, D, nin, nout);
     if (cost < best) {
       best = cost;
@@ -1543,7 +1549,6 @@ void with_capacity(int njobs, F&& f) {
   else if (njobs <= 8) f(std::integral_constant<int, 8>{});
   else f(std::integral_constant<int, kMaxJobs>{});
 }
-constexpr size_t kSmemCap = 200 * 1024;  // dynamic shared memory of a pass
 template <typename K>
 void allow_smem(K kern) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
@@ -1551,10 +1556,10 @@ void allow_smem(K kern) {
 
 int p1_terms(const AxisJob& J) { return (std::min(J.jhi, J.nin) + J.B - 1) / J.B; }
 // Shared memory of the passes (the twiddles, pass 1 also the inputs).
-size_t pass1_smem(const AxisJob& J, int P) {
+size_t pass1_smem(const AxisJob& J, int P, bool staged) {
   const int K = p1_terms(J), Kp = (K + 1) & ~1;
   const P1Shape s = p1_shape(J.A, J.B, P);
-  return sizeof(double) * (4 * (size_t)J.A + (size_t)Kp * s.G);
+  return sizeof(double) * ((staged ? 4 * (size_t)J.A : 0) + (size_t)Kp * s.G);
 }
 size_t pass2_smem(const AxisJob& J) { return sizeof(double) * ((size_t)J.D + 1); }
 size_t pass2_lines_smem(const AxisJob& J) { return sizeof(double) * 2 * 32 * (size_t)J.B; }
@@ -1582,7 +1587,8 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
     for (int nj : {1, 2, 4, 8, kMaxJobs})
       with_capacity(nj, [&](auto c) {
         constexpr int NJ = decltype(c)::value;
-        allow_smem(two_level_pass1<NJ>);
+        allow_smem(two_level_pass1<NJ, true>);
+        allow_smem(two_level_pass1<NJ, false>);
         allow_smem(two_level_pass2<NJ, 16>);
         allow_smem(two_level_pass2<NJ, 32>);
       });
@@ -1605,11 +1611,13 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   int P = 16;
   while (P > 2 && 2 * ctas1(P) > std::max(nsm, 1)) P /= 2;
   size_t smem1 = 0, smem2 = 0;
+  bool staged = true;
+  for (int i = 0; i < b.njobs; ++i) staged = staged && pass1_smem(b.job[i], P, true) <= kSmemCap;
   int total = 0;
   for (int i = 0; i < b.njobs; ++i) {
     const AxisJob& J = b.job[i];
     const P1Shape s = p1_shape(J.A, J.B, P);
-    smem1 = std::max(smem1, pass1_smem(J, P));
+    smem1 = std::max(smem1, pass1_smem(J, P, staged));
     b.start[i] = total;
     total += J.nlines * s.kblocks * s.jblocks;
   }
@@ -1617,7 +1625,8 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
   if (total > 0)
     with_capacity(b.njobs, [&](auto c) {
       constexpr int NJ = decltype(c)::value;
-      launch_pdl(two_level_pass1<NJ>, dim3(total), dim3(kP1Threads), smem1, st, shrink<NJ>(b), P);
+      launch_pdl(staged ? two_level_pass1<NJ, true> : two_level_pass1<NJ, false>, dim3(total), dim3(kP1Threads), smem1, st,
+                 shrink<NJ>(b), P);
     });
   // pass 2 with many lines per job: line groups share their staged twiddles; and
   // with any length whose whole table is over the shared memory (D > 25599), as

@@ -26,8 +26,13 @@ print(json.dumps(out))
 SIZES = [(12800, 3),   # D = 25599 on the dealiased grid: the last whose table fits
          (16385, 3),   # D = 16384 | 32769 = 331 x 99
          (25600, 1), (25601, 1), (25606, 1), (32769, 1)]
+# D = 4 x 3847, 4 x 4999, 4 x 5147 and 4 x 6553: the first level's table of 2 A
+# pairs with A on both sides of 5119
+WIDE = [(15389, 1), (19997, 1), (20589, 1), (26213, 1)]
 
 
-def test_long_axes(host_lib):
-    for r in run(host_lib, SCRIPT.replace("SIZES", repr(SIZES))):
+@pytest.mark.parametrize("sizes", [SIZES, WIDE], ids=["long", "wide"])
+def test_long_axes(host_lib, sizes):
+    for r in run(host_lib, SCRIPT.replace("SIZES", repr(sizes))):
+        assert r["one"] > 0, r
         assert r["pending"] == 0 and r["one"] == r["two"] and r["smem"] <= 200 * 1024, r
