@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(NT, NT == kFT ? HOSNWT_FFT_MIN_BLOCKS : 1)
   using T = typename std::conditional<DF, dfc, double2>::type;
   extern __shared__ __align__(128) double2 fsm[];
   __shared__ double red[kFWMax][kFMaxLines];
-  __shared__ T z0s[kFMaxLines / 2], a0s[kFMaxLines / 2];
+  __shared__ T z0s[kFMaxLines], a0s[kFMaxLines];  // one per sequence: double-float takes a line each
   __shared__ __align__(8) uint64_t tma_bar;
   int jb = 0;
   while (jb + 1 < b.njobs && (int)blockIdx.x >= b.start[jb + 1]) ++jb;
@@ -1798,6 +1798,20 @@ bool fft_tune_enabled() {
   return on && fft_df_enabled();
 }
 
+// HOSNWT_FFT_LAYOUT=threads,shift holds every double-float batch that can take
+// it at one of the tuner's layouts (a test of each, whatever the tuner likes)
+static FftLayout fft_forced_layout() {
+  static const FftLayout lay = [] {
+    FftLayout l;
+    const char* e = std::getenv("HOSNWT_FFT_LAYOUT");
+    if (e && (std::sscanf(e, "%d,%d", &l.nt, &l.pshift) != 2 || (l.nt != kFT && l.nt != kFTBig) || l.pshift < -2 ||
+              l.pshift > 1))
+      l = FftLayout{};
+    return fft_df_enabled() ? l : FftLayout{};
+  }();
+  return lay;
+}
+
 void fft_tune_record(bool on) { g_tune_recording = on; }
 
 int fft_tune_run(cudaStream_t st) {
@@ -1860,8 +1874,8 @@ int fft_tune_run(cudaStream_t st) {
 }
 
 void launch_fft_jobs(const AxisBatch& in, const FftPlanInfo* const* plan, const Tables& tb, cudaStream_t st) {
-  FftLayout lay;
-  if (fft_tune_enabled()) {
+  FftLayout lay = fft_forced_layout();
+  if (lay.nt == 0 && fft_tune_enabled()) {
     const std::string sig = fft_signature(in, plan);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_done.find(sig);
