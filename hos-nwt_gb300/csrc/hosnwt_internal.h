@@ -356,6 +356,7 @@ struct Tables {
   // sums use the scratch cs
   TcMat tc[kTcMats];
   int ntc = 0;
+  int tc_units = 0;          // buffers of sums that the scratch holds
 };
 
 // The plan of tb for J's length when the FFT pass should run J (a REDFT00 /
@@ -366,18 +367,27 @@ struct Tables {
 const FftPlanInfo* fft_choice(const AxisJob& J, const Tables& tb, double cost_other);
 // Launch the FFT passes of b's jobs, job i with plan[i].
 void launch_fft_jobs(const AxisBatch& b, const FftPlanInfo* const* plan, const Tables& tb, cudaStream_t st);
-// Tensor-core passes (tcx.cu).  build_tc_matrix makes a matrix on the device
-// (appended to `allocs`).  tc_choose sets AxisJob::tc of the requests that
+// Tensor-core passes (tcx.cu).  describe_tc_matrix gives the extents of a matrix,
+// build_tc_matrix makes it on the device (appended to `allocs`).  tc_choose sets AxisJob::tc of the requests that
 // should run there, given the time (us) of their passes elsewhere: jobs[p][i]
 // and alt[p][i] are pass p of request i, p = 0 the x and 1 the y pass, or a y
 // pass alone (npass = 1).  launch_tc_jobs runs the jobs of a batch (all x or
 // all y passes, every one with its matrix), false if one of them does not fit
 // the scratch.
-bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<long double>& quarter,
-                     double* scratch, std::vector<void*>& allocs, TcMat* out);
-// Scratch (doubles) that holds the digits of `first` lines of `second` points
-// for each of the given pairs, one at a time.
-long long tc_scratch_doubles(int nsm, const std::vector<std::pair<long long, int>>& lines);
+bool describe_tc_matrix(int D, int form, int sin_kind, double scale, int nout, TcMat* out);
+bool build_tc_matrix(TcMat* m, std::vector<long double>& quarter, double* scratch, std::vector<void*>& allocs);
+// What a batch of up to `most` requests like the given one (its pass p is passes[p],
+// as in tc_choose) needs: whether tc_choose takes any of them, and then the most
+// buffers of sums and bytes of digits.  `need` accumulates.
+struct TcNeed {
+  bool any = false;
+  long long units = 0, digits = 0;
+};
+void tc_need(const AxisJob* passes, const double* alt, int npass, const Tables& tb, int most, int held, TcNeed* need);
+long long tc_scratch_doubles(const TcNeed& need);
+// The same over the requests of a tank (xform.cu), `most` in its largest batch;
+// `lines`: the lines of its y passes that have no x pass.
+TcNeed tank_tc_need(const Tables& tb, int most, const std::vector<int>& lines);
 void tc_choose(AxisJob* const* jobs, const double* const* alt, int npass, int n, const Tables& tb);
 bool launch_tc_jobs(const AxisBatch& b, const Tables& tb, cudaStream_t st);
 // Layout tuning of the FFT passes: with recording on (this thread), launches

@@ -836,25 +836,8 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
     c.tb.cnt_cap = 4 * c.tb.nsm * 16;
     c.tb.part = dalloc<double>(c, (size_t)c.tb.part_cap);
     c.tb.cnt = dalloc<unsigned int>(c, (size_t)c.tb.cnt_cap);
-    // two-level pass scratch: up to kMaxJobs x-pass jobs over nd2 lines,
-    // B (A+1) 2 <= 2 (D+2) doubles per line for any factor pair
-    c.tb.cs_cap = (long long)kMaxJobs * std::max(nd2, n2) * 4LL * (std::max(nd1, n1) + 2);
-    // the tensor-core passes of a 3-D tank keep their digits and sums there:
-    // kMaxJobs fields of the dealiased grid, or the y lines of phiadd_SL
-    if (n2 > 1)
-      c.tb.cs_cap = std::max(c.tb.cs_cap, tc_scratch_doubles(c.tb.nsm, {{kMaxJobs * nd2, nd1}, {kMaxJobs * nd1, nd2},
-                                                                        {n1 * n3a, n2}}));
-    c.tb.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
-    // the wavemaker branch runs on its own stream with its own scratch
-    c.tb2 = c.tb;
-    c.tb2.part = dalloc<double>(c, (size_t)c.tb.part_cap);
-    c.tb2.cnt = dalloc<unsigned int>(c, (size_t)c.tb.cnt_cap);
-    c.tb2.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
-    // and so does the eta-power branch
-    c.tb3 = c.tb;
-    c.tb3.part = dalloc<double>(c, (size_t)c.tb.part_cap);
-    c.tb3.cnt = dalloc<unsigned int>(c, (size_t)c.tb.cnt_cap);
-    c.tb3.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
+    c.tb.cs_cap = 0;
+    c.tb.cs = nullptr;
   }
   c.tb.q_n1 = d.q_n1; c.tb.q_n2 = d.q_n2; c.tb.q_nd1 = d.q_nd1; c.tb.q_nd2 = d.q_nd2; c.tb.q_add = d.q_add;
   // FFT plans of the x and y lengths (passes over many lines: 3-D tanks)
@@ -868,22 +851,19 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
       if (build_fft_plan(D, c.allocs, &f)) c.tb.fft[c.tb.nfft++] = f;
     }
   }
-  // nothing is launched with an array that was refused; the matrices below may
-  // be, and what they find pending would be taken for their own
-  if (c.alloc_failed || cudaPeekAtLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "device allocation failed");
   // matrices of the tensor-core passes: F2S in cos and sin and S2F in cos
   // (what the right-hand side transforms), the S2F of the dealiased grid
-  // also truncated to the free-surface modes
+  // also truncated to the free-surface modes; none, and no scratch for them, in a
+  // tank none of whose passes would go there
   c.tb.ntc = 0;
+  TcNeed need;
   if (n2 > 1) {
-    std::vector<long double> quarter;
-    double* const tmp = c.tb.cs ? c.tb.cs + kTcMaxBytes / 8 : nullptr;  // behind the maxima and the error flag
     auto add = [&](int D, int form, int sin_kind, double scale, int nout) {
       for (int i = 0; i < c.tb.ntc; ++i) {
         const TcMat& m = c.tb.tc[i];
         if (m.D == D && m.form == form && m.sin_kind == sin_kind && m.scale == scale && nout <= m.nout) return;
       }
-      if (c.tb.ntc < kTcMats && build_tc_matrix(D, form, sin_kind, scale, nout, quarter, tmp, c.allocs, &c.tb.tc[c.tb.ntc])) ++c.tb.ntc;
+      if (c.tb.ntc < kTcMats && describe_tc_matrix(D, form, sin_kind, scale, nout, &c.tb.tc[c.tb.ntc])) ++c.tb.ntc;
     };
     for (int axis = 0; axis < 2; ++axis) {
       const int n = axis ? n2 : n1, nd = axis ? nd2 : nd1;
@@ -894,14 +874,43 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
       }
       if (nd > n) add(nd - 1, 1, 0, 2.0 * (1.0 / (nd - 1)), n);
     }
-    if (cudaStreamSynchronize(0) != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "transform matrices failed");
+    // the largest batch of a right-hand side has 8 (M = 2) to 16 fields (M = 11);
+    // y passes without an x pass: the wavemaker branch's
+    need = tank_tc_need(c.tb, std::min(M + 7, kMaxJobs), {n1, P.n3, n1 * n3a});
+    if (!need.any) c.tb.ntc = 0;
   }
+  // two-level pass scratch: up to kMaxJobs x-pass jobs over nd2 lines,
+  // B (A+1) 2 <= 2 (D+2) doubles per line for any factor pair; the tensor-core
+  // passes keep their digits and sums there
+  c.tb.cs_cap = (long long)kMaxJobs * std::max(nd2, n2) * 4LL * (std::max(nd1, n1) + 2);
+  if (need.any) c.tb.cs_cap = std::max(c.tb.cs_cap, tc_scratch_doubles(need));
+  c.tb.tc_units = (int)need.units;
+  c.tb.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
+  // the wavemaker branch and the eta-power branch run on their own streams with
+  // their own scratch
   for (Tables* t : {&c.tb2, &c.tb3}) {
-    t->ntc = c.tb.ntc;
-    for (int i = 0; i < c.tb.ntc; ++i) t->tc[i] = c.tb.tc[i];
-    t->q_n1 = d.q_n1; t->q_n2 = d.q_n2; t->q_nd1 = d.q_nd1; t->q_nd2 = d.q_nd2; t->q_add = d.q_add;
-    t->nfft = c.tb.nfft;
-    for (int i = 0; i < c.tb.nfft; ++i) t->fft[i] = c.tb.fft[i];
+    *t = c.tb;
+    t->part = dalloc<double>(c, (size_t)c.tb.part_cap);
+    t->cnt = dalloc<unsigned int>(c, (size_t)c.tb.cnt_cap);
+    t->cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
+  }
+  // nothing is launched with an array that was refused; the matrices below may
+  // be, and what they find pending would be taken for their own
+  if (c.alloc_failed || cudaPeekAtLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "device allocation failed");
+  if (c.tb.ntc > 0) {
+    std::vector<long double> quarter;
+    double* const tmp = c.tb.cs + kTcMaxBytes / 8;  // behind the maxima and the error flag
+    int built = 0;
+    for (int i = 0; i < c.tb.ntc; ++i) {
+      TcMat m = c.tb.tc[i];
+      if (build_tc_matrix(&m, quarter, tmp, c.allocs)) c.tb.tc[built++] = m;
+    }
+    c.tb.ntc = built;
+    for (Tables* t : {&c.tb2, &c.tb3}) {
+      t->ntc = built;
+      for (int i = 0; i < built; ++i) t->tc[i] = c.tb.tc[i];
+    }
+    if (cudaStreamSynchronize(0) != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "transform matrices failed");
   }
   if (cudaGetLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "upload failed");
   return HOSNWT_OK;

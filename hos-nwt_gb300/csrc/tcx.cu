@@ -1116,13 +1116,28 @@ int tc_mode() {
 }  // namespace
 
 // The matrix of one form of a pass of length D (see TcMat).  scale is the
-// interior output scale times the interior input weight; quarter holds the first
-// quarter turn's cosines, filled as they are asked for (the forms of a length
-// share them); the table of entries passes through `scratch`.  The matrix is
-// complete once the default stream is.
-bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std::vector<long double>& quarter,
-                     double* scratch, std::vector<void*>& allocs, TcMat* out) {
-  if (D < 8 || D > kTcMaxD || !scratch) return false;
+// interior output scale times the interior input weight.
+bool describe_tc_matrix(int D, int form, int sin_kind, double scale, int nout, TcMat* out) {
+  if (D < 8 || D > kTcMaxD) return false;
+  *out = TcMat{};
+  out->D = D;
+  out->form = form;
+  out->sin_kind = sin_kind;
+  out->scale = scale;
+  out->nout = form == 0 ? D + 1 : nout;
+  out->nrows = form == 0 ? D / 2 + 1 : (nout + 1) / 2;
+  out->kp = pad_k(D / 2 + 1);
+  return true;
+}
+
+// Its digits on the device.  quarter holds the first quarter turn's cosines,
+// filled as they are asked for (the forms of a length share them); the table of
+// entries passes through `scratch`.  The matrix is complete once the default
+// stream is.
+bool build_tc_matrix(TcMat* out, std::vector<long double>& quarter, double* scratch, std::vector<void*>& allocs) {
+  const int D = out->D, form = out->form, sin_kind = out->sin_kind;
+  const double scale = out->scale;
+  if (!scratch) return false;
   int ew = 0;
   const long double c = frexpl((long double)scale, &ew);  // scale = c 2^ew, c in [1/2, 1)
   const long double pi = 3.141592653589793238462643383279502884L;
@@ -1145,8 +1160,7 @@ bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std:
     for (int s = 0; s < 5; ++s) t[s] = bf16_bits(d[s]);
     t[5] = bf16_bits(d[4] - bf16_float(t[4]));
   }
-  const int nrows = form == 0 ? D / 2 + 1 : (nout + 1) / 2;
-  const int kp = pad_k(D / 2 + 1);
+  const int nrows = out->nrows, kp = out->kp;
   void* mat = nullptr;
   if (cudaMalloc(&mat, (size_t)2 * kS * nrows * kp * 2) != cudaSuccess) {
     cudaGetLastError();  // this refusal: the job keeps its other pass
@@ -1156,22 +1170,13 @@ bool build_tc_matrix(int D, int form, int sin_kind, double scale, int nout, std:
   if (cudaMemcpy(scratch, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice) != cudaSuccess) return false;
   k_tc_matrix<<<1024, 256>>>((const uint4*)scratch, (__nv_bfloat16*)mat, D, form, nrows, kp);
   if (cudaPeekAtLastError() != cudaSuccess) return false;  // left for the caller
-  out->D = D;
-  out->form = form;
-  out->sin_kind = sin_kind;
-  out->scale = scale;
-  out->nout = form == 0 ? D + 1 : nout;
-  out->nrows = nrows;
-  out->kp = kp;
   out->ew = ew;
   out->dev = mat;
   return true;
 }
 
-long long tc_scratch_doubles(int nsm, const std::vector<std::pair<long long, int>>& lines) {
-  long long most = 0;
-  for (const auto& l : lines) most = std::max(most, l.first * (pad_k((l.second + 1) / 2) * 4LL * kS + 4));
-  return kTcMaxBytes / 8 + nsm * kUnitsPerSm * kSums + most / 8 + 512 * kMaxJobs;
+long long tc_scratch_doubles(const TcNeed& need) {
+  return kTcMaxBytes / 8 + need.units * kSums + need.digits / 8 + 512 * kMaxJobs;
 }
 
 const TcMat* tc_matrix_of(const AxisJob& J, const Tables& tb) {
@@ -1255,12 +1260,48 @@ void tc_choose(AxisJob* const* jobs, const double* const* alt, int npass, int n,
   }
   if (chosen.empty()) return;
   for (int p = 0; p < npass; ++p) {
-    tc += 17.0 + best_split(shapes[p], nsm, (long long)nsm * kUnitsPerSm).cycles / 1900.0;
+    tc += 17.0 + best_split(shapes[p], nsm, tb.tc_units).cycles / 1900.0;
     other += 8.0;
   }
   if (tc > other && tc_mode() != 2) return;
   for (int i : chosen)
     for (int p = 0; p < npass; ++p) jobs[p][i].tc = mat[(size_t)p * n + i];
+}
+
+// A batch of one, a few and `most` requests of one kind: what a request gains does
+// not fall with their number (the launches are shared), and in a mixed batch no
+// kind gains more than alone.  The buffers of sums are those of kMaxJobs requests cut
+// as far as best_split cuts, or the kBufs of every CTA, and at most kUnitsPerSm per
+// SM; the digits those of `held` requests (a batch of more goes in parts).
+void tc_need(const AxisJob* passes, const double* alt, int npass, const Tables& tb, int most, int held, TcNeed* need) {
+  const int nsm = std::max(tb.nsm, 1);
+  Tables full = tb;
+  full.tc_units = nsm * kUnitsPerSm;
+  bool any = false;
+  for (int q : {1, (most + 1) / 2, most}) {
+    std::vector<AxisJob> j[2];
+    std::vector<double> a[2];
+    AxisJob* jobs[2] = {};
+    const double* alts[2] = {};
+    for (int p = 0; p < npass; ++p) {
+      j[p].assign(q, passes[p]);
+      a[p].assign(q, alt[p]);
+      jobs[p] = j[p].data();
+      alts[p] = a[p].data();
+    }
+    tc_choose(jobs, alts, npass, q, full);
+    if (!j[0][0].tc) continue;
+    any = true;
+    for (int p = 0; p < npass; ++p) {
+      const TcMat& m = *j[p][0].tc;
+      const GroupShape one = shape_of(passes[p], m, passes[p].nlines);
+      const long long tiles = (long long)kMaxJobs * one.tiles;
+      const long long units = std::max(tiles * std::min(8, one.nkb) * one.np, kBufs * std::min<long long>(nsm, tiles));
+      need->units = std::max(need->units, std::min<long long>(units, full.tc_units));
+      need->digits = std::max(need->digits, (long long)held * passes[p].nlines * (terms_of(passes[p], m) * 4LL * kS + 4));
+    }
+  }
+  need->any = need->any || any;
 }
 
 bool launch_tc_jobs(const AxisBatch& in, const Tables& tb, cudaStream_t st) {
@@ -1269,7 +1310,8 @@ bool launch_tc_jobs(const AxisBatch& in, const Tables& tb, cudaStream_t st) {
   const bool ymode = in.njobs > 0 && in.job[0].in_sk != 1;
   char* const scratch = reinterpret_cast<char*>(tb.cs) + kTcMaxBytes;  // after the maxima
   const long long cap = tb.cs_cap * (long long)sizeof(double) - kTcMaxBytes;
-  const long long sum_cap = (long long)tb.nsm * kUnitsPerSm;  // buffers of sums
+  const long long sum_cap = tb.tc_units;  // buffers of sums
+  if (sum_cap < kBufs) return false;
   const long long stash_bytes = sum_cap * kSums * 8;
   // groups of jobs with the same matrix and extents
   std::vector<std::vector<int>> groups;
@@ -1443,7 +1485,9 @@ bool launch_tc_jobs(const AxisBatch& in, const Tables& tb, cudaStream_t st) {
       t.failed = B.failed;
       if (ymode) launch_pdl(k_tc_digits_y<NJ>, dim3(dblocks), dim3(kDgThreads), kDgySmem, st, d);
       else launch_pdl(k_tc_digits_x<NJ>, dim3(dblocks), dim3(kDgThreads), 0, st, d);
-      launch_pdl(k_tc_pass<NJ>, dim3(std::min(B.nunits, tb.nsm)), dim3(kThreads), kPassSmem, st, t);
+      // whole tiles: kBufs buffers per CTA
+      const int ctas = B.split ? tb.nsm : (int)std::min<long long>(tb.nsm, sum_cap / kBufs);
+      launch_pdl(k_tc_pass<NJ>, dim3(std::min(B.nunits, ctas)), dim3(kThreads), kPassSmem, st, t);
       if (B.split) launch_pdl(k_tc_finish<NJ>, dim3(ntiles * (kBN / kOutCols)), dim3(kOutWarps * 32), 0, st, t);
     });
   }

@@ -2287,6 +2287,45 @@ void launch_ordered(const XfReq* reqs, const int* idx, int n, const Tables& tb, 
 
 }  // namespace
 
+TcNeed tank_tc_need(const Tables& tb, int most, const std::vector<int>& lines) {
+  TcNeed need;
+  auto look = [&](int Nx, int Ny, int dir, int nin1, int nin2, int nout1, int nout2) {
+    AxisJob p[2] = {};
+    set_kind(p[0], axis_kind(0, dir, 0), Nx, nullptr);
+    set_kind(p[1], axis_kind(0, dir, 0), Ny, nullptr);
+    p[0].nin = nin1;
+    p[0].nout = nout1;
+    p[0].nlines = nin2;
+    p[0].in_sk = 1;
+    p[0].in_sl = nin1;
+    p[1].nin = nin2;
+    p[1].nout = nout2;
+    p[1].nlines = p[1].in_sk = nout1;
+    p[1].in_sl = 1;
+    p[0].gscale = p[1].gscale = 1.0;
+    const double alt[2] = {pass_time(p[0], tb, false), pass_time(p[1], tb, true)};
+    tc_need(p, alt, 2, tb, most, kMaxJobs, &need);
+    tc_need(p + 1, alt + 1, 1, tb, most, kMaxJobs, &need);  // the x pass without a matrix (sin kinds)
+  };
+  for (int dir : {1, -1}) {
+    look(tb.n1, tb.n2, dir, tb.n1, tb.n2, tb.n1, tb.n2);
+    look(tb.nd1, tb.nd2, dir, tb.nd1, tb.nd2, tb.nd1, tb.nd2);
+  }
+  look(tb.nd1, tb.nd2, 1, tb.nd1, tb.nd2, tb.n1, tb.n2);
+  look(tb.nd1, tb.nd2, -1, tb.n1, tb.n2, tb.nd1, tb.nd2);
+  for (int n : lines) {
+    AxisJob y{};
+    set_kind(y, K_C1_F2S, tb.n2, nullptr);
+    y.nin = y.nout = tb.n2;
+    y.nlines = y.in_sk = n;
+    y.in_sl = 1;
+    y.gscale = 1.0;
+    const double alt = pass_time(y, tb, true);
+    tc_need(&y, &alt, 1, tb, most, 1, &need);
+  }
+  return need;
+}
+
 void launch_transforms(const XfReq* reqs, int nreq, const Tables& tb, double* const* tmp,
                        cudaStream_t st) {
   // x then y for every request.  (Running the y pass first, where it takes
