@@ -956,7 +956,7 @@ __global__ void __launch_bounds__(kP2Threads) two_level_pass2(const AxisBatchT<N
   }
 }
 
-// pass 2 for launches with many lines (the x passes of 3-D tanks):
+// pass 2 for lengths whose quarter-wave table is over the shared memory:
 // CTA = (job, 32 outputs, group of lpc lines).  The B x 32 twiddle tile is
 // staged once for the group; each warp takes lines in turn and sums all of
 // their j2 terms, so no cross-warp reduction is needed.
@@ -1519,7 +1519,7 @@ void pick_factors(int D, int nin, int nout, int* Aout, int* Bout) {
   for (int A = 2; A <= D / 2; ++A) {
     if (D % A) continue;
     const int B = D / A;
-    if (B < 2 || B > 256) continue;  // pass 2 of many lines stages B x 32 twiddle pairs
+    if (B < 2 || B > 256) continue;  // two_level_pass2_lines stages B x 32 twiddle pairs
     if (8LL * (A + 2) > (long long)kSmemCap) continue;  // pass 1's inputs
     const double cost = x_two_level_cost(A, B, D, nin, nout);
     if (cost < best) {
@@ -1628,16 +1628,14 @@ void launch_two_level(AxisBatch& b, int nsm, bool early, cudaStream_t st) {
       launch_pdl(staged ? two_level_pass1<NJ, true> : two_level_pass1<NJ, false>, dim3(total), dim3(kP1Threads), smem1, st,
                  shrink<NJ>(b), P);
     });
-  // pass 2 with many lines per job: line groups share their staged twiddles; and
-  // with any length whose whole table is over the shared memory (D > 25599), as
-  // these hold B x 32 of them (128 KB at most)
-  int minl = 1 << 30;
+  // Pass 2 gathers from a staged quarter-wave table whatever the lines.  (Groups of
+  // lines that shared a staged tile of B x 32 pairs took 16 lines and more: 16 of 1024
+  // points 74 us for both passes, 14 with the gather; 513 of 1025 points 355 and 124;
+  // nowhere less, from 66 to 8193 points.)  Lengths whose table is over the shared
+  // memory (D > 25599) keep the tiles, of 128 KB at most.
   size_t table = 0;
-  for (int i = 0; i < b.njobs; ++i) {
-    minl = std::min(minl, b.job[i].nlines);
-    table = std::max(table, pass2_smem(b.job[i]));
-  }
-  if (minl >= 16 || table > kSmemCap) {
+  for (int i = 0; i < b.njobs; ++i) table = std::max(table, pass2_smem(b.job[i]));
+  if (table > kSmemCap) {
     static PerDeviceOnce attr_l;
     attr_l.run([&] {
       for (int nj : {1, 2, 4, 8, kMaxJobs})

@@ -1,0 +1,34 @@
+"""Which kernels the context-free transform launches, by length and lines, on
+both sides of its rules."""
+import pytest
+
+from host_lib import link, run
+
+
+@pytest.fixture(scope="module")
+def host_lib():
+    return link()
+
+
+SCRIPT = r"""
+out = []
+for n, lines in CALLS:
+    lib.host_cudart_reset()
+    hosnwt.transform_noalloc(1, "cos", n, lines, 1 << 30, 1 << 31, 0)
+    out.append({"n": n, "lines": lines, "pending": lib.host_cudart_pending(),
+                **{k: launches(k)[0] for k in ("two_level_pass1", "two_level_pass2_lines", "two_level_pass2", "direct_pass",
+                                               "axis_pass_lanes_k")}})
+print(json.dumps(out))
+"""
+
+
+def _run(host_lib, calls):
+    return run(host_lib, SCRIPT.replace("CALLS", repr(calls)))
+
+
+def test_many_lines_gather_their_twiddles(host_lib):
+    """16 lines and more of a length that factors: the pass that shares a staged
+    tile of twiddles took five times as long (1024 points, 16 lines)."""
+    for r in _run(host_lib, [(1024, 15), (1024, 16), (723, 32), (1026, 24), (513, 100), (2052, 16)]):
+        assert r["pending"] == 0 and r["two_level_pass1"] == r["two_level_pass2"] > 0, r
+        assert r["two_level_pass2_lines"] == 0, r
