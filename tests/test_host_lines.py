@@ -32,3 +32,10 @@ def test_many_lines_gather_their_twiddles(host_lib):
     for r in _run(host_lib, [(1024, 15), (1024, 16), (723, 32), (1026, 24), (513, 100), (2052, 16)]):
         assert r["pending"] == 0 and r["two_level_pass1"] == r["two_level_pass2"] > 0, r
         assert r["two_level_pass2_lines"] == 0, r
+
+
+def test_long_lines_go_in_chunks(host_lib):
+    """16 lines and more of 7900 points and up, of which fewer than 16 fit the fixed
+    scratch at a time: two levels in chunks, not direct sums over every pair."""
+    for r, want in zip(_run(host_lib, [(8193, 15), (8193, 16), (8193, 46), (16385, 4), (16385, 8), (8161, 33)]), (1, 2, 4, 1, 2, 3)):
+        assert r["pending"] == 0 and r["axis_pass_lanes_k"] == 0 and r["two_level_pass1"] == want, r
