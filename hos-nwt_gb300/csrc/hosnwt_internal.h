@@ -325,9 +325,9 @@ struct TcMat {
 };
 constexpr int kTcMaxD = 6200;  // the fixed-point sums of tcx.cu hold two parities of this many terms
 constexpr int kTcMats = 16;
-// room for the maxima of kMaxJobs x passes and an error flag at the start of
-// the scratch; the two-level passes keep off it
-constexpr long long kTcMaxBytes = ((long long)kMaxJobs * (kTcMaxD + 8) * 4 + 64 + 1023) / 1024 * 1024;
+// room for the maxima of kMaxJobs x passes at the start of the scratch; the
+// two-level passes keep off it
+constexpr long long kTcMaxBytes = ((long long)kMaxJobs * (kTcMaxD + 8) * 4 + 1023) / 1024 * 1024;
 
 struct Tables {
   int n1, n2, nd1, nd2, n3_add;
@@ -357,6 +357,8 @@ struct Tables {
   TcMat tc[kTcMats];
   int ntc = 0;
   int tc_units = 0;          // buffers of sums that the scratch holds
+  unsigned* tc_failed = nullptr;   // set by a pass whose wait ran out; device memory
+  unsigned* tc_expired = nullptr;  // and for the host; page-locked host memory
 };
 
 // The plan of tb for J's length when the FFT pass should run J (a REDFT00 /

@@ -885,6 +885,8 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
   c.tb.cs_cap = (long long)kMaxJobs * std::max(nd2, n2) * 4LL * (std::max(nd1, n1) + 2);
   if (need.any) c.tb.cs_cap = std::max(c.tb.cs_cap, tc_scratch_doubles(need));
   c.tb.tc_units = (int)need.units;
+  c.tb.tc_failed = d.tc_failed;
+  c.tb.tc_expired = d.tc_expired;
   c.tb.cs = dalloc<double>(c, (size_t)c.tb.cs_cap);
   // the wavemaker branch and the eta-power branch run on their own streams with
   // their own scratch
@@ -899,7 +901,7 @@ int setup(Ctx& c, const char* wave_dir, const double* probes_xy, int nprobes) {
   if (c.alloc_failed || cudaPeekAtLastError() != cudaSuccess) return fail(c, HOSNWT_ERR_CUDA, "device allocation failed");
   if (c.tb.ntc > 0) {
     std::vector<long double> quarter;
-    double* const tmp = c.tb.cs + kTcMaxBytes / 8;  // behind the maxima and the error flag
+    double* const tmp = c.tb.cs + kTcMaxBytes / 8;  // behind the maxima
     int built = 0;
     for (int i = 0; i < c.tb.ntc; ++i) {
       TcMat m = c.tb.tc[i];
@@ -976,6 +978,9 @@ int alloc_device(Ctx& c) {
   const size_t nparts = 10 * ((S + 255) / 256) + (std::max(nB, nN) + 63) / 64 + 1024;
   d.part = dalloc<double>(c, nparts);
   d.counter = dalloc<unsigned int>(c, 16);
+  d.tc_failed = dalloc<unsigned int>(c, 1);
+  if (cudaMallocHost((void**)&d.tc_expired, sizeof(unsigned)) != cudaSuccess) return 1;
+  *d.tc_expired = 0;
   if (cudaMallocHost((void**)&d.host_sc, SC_COUNT * sizeof(double)) != cudaSuccess) return 1;
   std::memset(d.host_sc, 0, SC_COUNT * sizeof(double));
   // staging of the drop-in step: eta, phis, the eight arrays from a_add_1
@@ -1001,6 +1006,8 @@ void free_device(Ctx& c) {
   for (void* p : c.allocs)
     if (p) cudaFree(p);
   c.allocs.clear();
+  if (c.d.tc_expired) cudaFreeHost(c.d.tc_expired);
+  c.d.tc_expired = nullptr;
   if (c.d.host_sc) cudaFreeHost(c.d.host_sc);
   c.d.host_sc = nullptr;
   if (c.d.host_io) cudaFreeHost(c.d.host_io);
@@ -1029,13 +1036,25 @@ struct hosnwt_ctx {
   hos::Ctx c;
 };
 
+// A wait of a tensor-core pass that ran out since the last look (the stream has
+// been synchronised): its outputs are NaN, the call reports it and the next starts
+// afresh.
+static int pass_check(Ctx& c, const char* what) {
+  volatile unsigned* const f = c.d.tc_expired;
+  if (!f || *f == 0) return HOSNWT_OK;
+  *f = 0;
+  cudaMemset(c.d.tc_failed, 0, sizeof(unsigned));
+  c.err = std::string(what) + ": a wait of a transform pass ran out";
+  return HOSNWT_ERR_CUDA;
+}
+
 static int cuda_check(Ctx& c, const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     c.err = std::string(what) + ": " + cudaGetErrorString(e);
     return HOSNWT_ERR_CUDA;
   }
-  return HOSNWT_OK;
+  return pass_check(c, what);
 }
 
 // Capture the step graph.  The first capture records the FFT batches that
@@ -1189,6 +1208,7 @@ static int run_step(Ctx& c, double t_o, double h_loc, double* err) {
   c.n_rhs += 5;
   const double e = c.d.host_sc[SC_ERR];
   if (err) *err = e;
+  if (const int rcp = pass_check(c, "step")) return rcp;
   if (!std::isfinite(e)) {
     c.err = "non-finite error estimate";
     return HOSNWT_ERR_NAN;
@@ -1427,6 +1447,7 @@ static int finish_loop(Ctx& c, double* h_rk_io, int* n_acc, int* n_rej) {
   *h_rk_io = b.h_rk;
   if (n_acc) *n_acc = b.n_acc;
   if (n_rej) *n_rej = b.n_rej;
+  if (const int rcp = pass_check(c, "advance")) return rcp;
   if (b.status == 1) {
     c.err = "non-finite error estimate";
     return HOSNWT_ERR_NAN;
@@ -1895,6 +1916,7 @@ extern "C" int hosnwt_advance_many(hosnwt_ctx* const* ctxs, int n, const double*
       if (q != cudaSuccess) { rc = cuda_check(c, "step"); break; }
       c.n_rhs += 5;
       const double error = c.d.host_sc[SC_ERR];
+      if ((rc = pass_check(c, "step"))) break;
       if (!std::isfinite(error)) {
         c.err = "non-finite error estimate";
         rc = HOSNWT_ERR_NAN;

@@ -102,6 +102,8 @@ struct Dev {
   unsigned int *counter = nullptr;
   double *probe_out = nullptr;
   double *host_sc = nullptr;    // pinned mirror of the scalar slots
+  unsigned *tc_failed = nullptr;   // a tensor-core pass had a wait run out (device)
+  unsigned *tc_expired = nullptr;  // the same, pinned: read where the host has synchronised
   double *host_io = nullptr;    // pinned staging of hosnwt_runge4_adapt2's arrays
 };
 

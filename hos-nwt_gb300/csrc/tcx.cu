@@ -100,7 +100,8 @@ struct TcBatchT {
   // per unit; k_tc_finish adds them up and writes the outputs).
   int split;
   long long* sums;              // [buffer][output][line]
-  unsigned* failed;             // split: set when a wait ran out
+  unsigned* failed;             // set when a wait ran out: k_tc_finish writes NaN
+  unsigned* expired;            // the same for the host (page-locked host memory)
 };
 using TcBatch = TcBatchT<kMaxJobs>;
 
@@ -843,14 +844,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
     double* stage = reinterpret_cast<double*>(base + kStages * kStageBytes) + quad * 2 * 32 * kStageRow;
     int ph = 0;
     bool ok = true;
-    for (int u = b.split ? b.nunits : (int)blockIdx.x; u < b.nunits && ok; u += gridDim.x) {
+    // once a wait has run out, NaN to every later tile of the CTA, without waiting
+    for (int u = b.split ? b.nunits : (int)blockIdx.x; u < b.nunits; u += gridDim.x) {
       const Unit w = unit(u);
-      for (int p = 0; p < w.np; ++p)
+      for (int p = 0; p < w.np && ok; ++p)
         if (!mbar_wait(&sum_full[(ph + p) % kBufs], (unsigned)(((ph + p) / kBufs) & 1))) ok = false;
       const long long* sums = b.sums + (long long)blockIdx.x * kBufs * kSums + quad * 32 + lane;
       put_outputs(b, w, quad, lane, sums + (ph % kBufs) * kSums, sums + ((ph + 1) % kBufs) * kSums, 1, stage, ok, 0, kBN);
       __syncwarp();
-      if (lane == 0)
+      if (lane == 0 && ok)  // else no buffer is given back: another output warp may be reading it
         for (int p = 0; p < w.np; ++p) mbar_arrive(&sum_empty[(ph + p) % kBufs]);
       ph += w.np;
     }
@@ -930,7 +932,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (abort_flag && threadIdx.x == 0) {
-    *b.failed = 1;  // k_tc_finish then writes NaN
+    *b.failed = 1;
+    *b.expired = 1;
+    __threadfence_system();
     // a wait ran out: let the loads in flight land before the CTA exits
     for (int i = n_used; i < n_loaded; ++i) (void)mbar_wait(&full_bar[i % kStages], (unsigned)((i / kStages) & 1));
     if (n_used > 0) (void)mbar_wait(&empty_bar[(n_used - 1) % kStages], (unsigned)(((n_used - 1) / kStages) & 1));
@@ -1341,7 +1345,8 @@ bool launch_tc_jobs(const AxisBatch& in, const Tables& tb, cudaStream_t st) {
     TcBatch B{};
     DgBatch Dg{};
     B.sums = reinterpret_cast<long long*>(scratch);
-    B.failed = reinterpret_cast<unsigned*>(scratch - 64);
+    B.failed = tb.tc_failed;
+    B.expired = tb.tc_expired;
     int ntiles = 0;
     long long used = (stash_bytes + 1023) / 1024 * 1024;
     int nj = 0, dblocks = 0;
@@ -1483,6 +1488,7 @@ bool launch_tc_jobs(const AxisBatch& in, const Tables& tb, cudaStream_t st) {
       t.split = B.split;
       t.sums = B.sums;
       t.failed = B.failed;
+      t.expired = B.expired;
       if (ymode) launch_pdl(k_tc_digits_y<NJ>, dim3(dblocks), dim3(kDgThreads), kDgySmem, st, d);
       else launch_pdl(k_tc_digits_x<NJ>, dim3(dblocks), dim3(kDgThreads), 0, st, d);
       // whole tiles: kBufs buffers per CTA

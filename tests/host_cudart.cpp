@@ -29,15 +29,14 @@ std::map<const void*, std::string>& names() {
 }
 std::map<const void*, size_t> g_smem_limit;
 std::map<void*, size_t> g_live;
+std::map<size_t, void*> g_pinned;  // the last page-locked block of each size
 std::vector<Launch> g_launches;
 size_t g_bytes = 0, g_peak = 0;
 int g_mallocs = 0, g_refuse = 0, g_refusals = 0;
 size_t g_at_refusal = 0;  // launches before the refused allocation
 bool g_capturing = false;
 int g_captured = 0;
-std::string g_fail_launch, g_watch;
-int g_watch_arg = 0;
-void* g_watched = nullptr;
+std::string g_fail_launch;
 cudaError_t g_last = cudaSuccess;
 
 cudaError_t ret(cudaError_t e) {
@@ -46,7 +45,7 @@ cudaError_t ret(cudaError_t e) {
 }
 constexpr size_t kSmemDefault = 48 * 1024, kSmemMost = 227 * 1024;
 
-cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t smem, void** args) {
+cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t smem) {
   const auto it = names().find(f);
   const std::string name = it == names().end() ? "?" : it->second;
   const auto lim = g_smem_limit.find(f);
@@ -55,7 +54,6 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t smem, void** arg
       grid.z > 65535u || block.x * block.y * block.z > 1024u || block.x == 0)
     return ret(cudaErrorInvalidValue);
   if (!g_fail_launch.empty() && name.find(g_fail_launch) != std::string::npos) return ret(cudaErrorLaunchOutOfResources);
-  if (!g_watch.empty() && name.find(g_watch) != std::string::npos) g_watched = *(void**)args[g_watch_arg];
   g_launches.push_back({name, grid, block, smem, g_capturing});
   if (g_capturing) ++g_captured;
   return cudaSuccess;
@@ -83,13 +81,16 @@ void host_cudart_reset() {
 }
 void host_cudart_refuse(int nth) { g_refuse = nth; }  // the nth cudaMalloc from the reset on fails; 0: none
 void host_cudart_fail_launch(const char* part) { g_fail_launch = part; }
-// the value of a pointer argument of the kernels whose name has `part`
-void host_cudart_watch(const char* part, int arg) {
-  g_watch = part;
-  g_watch_arg = arg;
-  g_watched = nullptr;
+void* host_cudart_pinned(long long size) {
+  const auto it = g_pinned.find((size_t)size);
+  return it == g_pinned.end() ? nullptr : it->second;
 }
-void* host_cudart_watched() { return g_watched; }
+int host_cudart_blocks(long long size, void** out, int most) {  // live device arrays of this size
+  int n = 0;
+  for (const auto& b : g_live)
+    if (b.second == (size_t)size && n < most) out[n++] = b.first;
+  return n;
+}
 int host_cudart_mallocs() { return g_mallocs; }
 int host_cudart_refusals() { return g_refusals; }
 long long host_cudart_bytes() { return (long long)g_bytes; }
@@ -142,11 +143,11 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) {
   *k = (cudaKernel_t)f;
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t) {
-  return launch((const void*)k, grid, block, smem, args);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void**, size_t smem, cudaStream_t) {
+  return launch((const void*)k, grid, block, smem);
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
-  return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, args);
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+  return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
@@ -211,6 +212,7 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaMallocHost(void** p, size_t n) {
   *p = calloc(1, n ? n : 1);
+  g_pinned[n] = *p;
   return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {

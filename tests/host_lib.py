@@ -23,7 +23,9 @@ import hosnwt, workloads
 lib = hosnwt.load_library(LIB)
 for f in ("host_cudart_bytes", "host_cudart_peak"):
     getattr(lib, f).restype = ctypes.c_longlong
-lib.host_cudart_watched.restype = ctypes.c_void_p
+lib.host_cudart_pinned.restype = ctypes.c_void_p
+lib.host_cudart_pinned.argtypes = [ctypes.c_longlong]
+lib.host_cudart_blocks.argtypes = [ctypes.c_longlong, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]
 
 def tank(n1, n2, n3, M, p1, p2=1, wmk=1, icase=2, **kw):
     if icase == 1:
