@@ -2376,6 +2376,24 @@ double measure_fp64_peak_gflops() {
 
 bool lines_direct(int n, int nlines) { return nlines <= kDirMaxLines && n - 1 <= kDirMaxD; }
 
+// Lines of a launch of direct sums.  Its tiles of 32 outputs go over the SMs in whole
+// waves, while 16 lines at a time leave a rest whose sums are cut over idle SMs:
+// 17 lines of 3000 points 344 us in one launch, 318 in two; 32 lines 568 and 576.
+// The waves of both, and the chunks where they save a fiftieth.
+int direct_lines(int D, int nlines, int nsm) {
+  constexpr int kChunk = 16;
+  if (nlines <= kChunk) return nlines;
+  auto waves = [&](int lines) {
+    const long long tiles = (long long)lines * ((D / 2 + 1 + 31) / 32), target = 4LL * nsm;
+    const int cut = tiles > 0 && tiles < target && D - 1 > 512
+                        ? std::min((int)((target + tiles - 1) / tiles), (D - 1 + 255) / 256) : 1;
+    return (double)((tiles * cut + nsm - 1) / nsm) / cut;
+  };
+  const double launch = 0.1;  // of a wave, for the last launch
+  const double chunks = nlines / kChunk * waves(kChunk) + (nlines % kChunk ? waves(nlines % kChunk) + launch : 0.0);
+  return chunks < 0.98 * waves(nlines) ? kChunk : nlines;
+}
+
 // nlines contiguous lines of n points (no context): two-level passes in chunks
 // that fit the scratch tb.part where the length factors, else the direct sums.
 void launch_lines(const Tables& tb, int dir, int cs, int n, int nlines, const double* in, double* out,
@@ -2393,7 +2411,7 @@ void launch_lines(const Tables& tb, int dir, int cs, int n, int nlines, const do
   // chunks of four lines and more: what is left to a last chunk of fewer is as
   // cheap (16 lines of 8193 points: 2.2 ms by the direct sums, 0.1 ms in chunks of 15)
   const bool two = chunk >= 4;
-  const int step = two ? (int)std::min<long long>(chunk, nlines) : nlines;
+  const int step = two ? (int)std::min<long long>(chunk, nlines) : direct_lines(J.D, nlines, tb.nsm);
   for (int l0 = 0; l0 < nlines; l0 += step) {
     AxisBatch b{};
     b.njobs = 1;

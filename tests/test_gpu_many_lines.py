@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 CALLS = [(2052, 64), (2052, 72), (2052, 130), (1024, 15), (1024, 16), (1024, 17), (723, 48), (66, 513),
          (1300, 9), (1300, 40), (3000, 17), (3000, 24), (4202, 9), (4202, 17), (5000, 20), (600, 9), (515, 20),
-         (8193, 15), (8193, 16), (8193, 33), (4097, 3), (2048, 2), (1024, 1)]
+         (8193, 15), (8193, 16), (8193, 33), (4097, 3), (2048, 2), (1024, 1), (3000, 20)]
 
 
 @pytest.mark.parametrize("direction,cs", [(1, "cos"), (-1, "cos"), (1, "sin"), (-1, "sin")])

@@ -39,3 +39,11 @@ def test_long_lines_go_in_chunks(host_lib):
     scratch at a time: two levels in chunks, not direct sums over every pair."""
     for r, want in zip(_run(host_lib, [(8193, 15), (8193, 16), (8193, 46), (16385, 4), (16385, 8), (8161, 33)]), (1, 2, 4, 1, 2, 3)):
         assert r["pending"] == 0 and r["axis_pass_lanes_k"] == 0 and r["two_level_pass1"] == want, r
+
+
+def test_direct_sums_of_a_wave_and_a_rest(host_lib):
+    """A few lines over 16 of a length that does not factor: a launch of 16 and one
+    of the rest, not a last wave that is nearly empty; whole waves in one launch."""
+    for r, want in zip(_run(host_lib, [(3000, 17), (3000, 20), (4202, 17), (3000, 16), (3000, 32), (1300, 40), (600, 300)]),
+                       (2, 2, 2, 1, 1, 1, 1)):
+        assert r["pending"] == 0 and r["axis_pass_lanes_k"] + r["direct_pass"] == want, r
