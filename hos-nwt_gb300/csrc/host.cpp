@@ -1042,9 +1042,11 @@ struct hosnwt_ctx {
 static int pass_check(Ctx& c, const char* what) {
   volatile unsigned* const f = c.d.tc_expired;
   if (!f || *f == 0) return HOSNWT_OK;
+  const bool lost = *f == 2;
   *f = 0;
   cudaMemset(c.d.tc_failed, 0, sizeof(unsigned));
   c.err = std::string(what) + ": a wait of a transform pass ran out";
+  if (lost) c.err += " and its products never finished: the CUDA context must not be used further";
   return HOSNWT_ERR_CUDA;
 }
 

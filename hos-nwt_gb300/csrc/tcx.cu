@@ -711,9 +711,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[3], acc_empty[3];  // levels 0-1, 2-3, 4-5
-  __shared__ uint64_t sum_full[kBufs], sum_empty[kBufs];
+  __shared__ uint64_t sum_full[kBufs], sum_empty[kBufs], mma_done;
   __shared__ uint32_t tmem_base;
-  __shared__ volatile int abort_flag;
+  __shared__ volatile int abort_flag, keep_tmem;
   __shared__ volatile int n_loaded, n_used;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -729,7 +729,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
       mbar_init(&sum_full[s], kDrainWarps);
       mbar_init(&sum_empty[s], kOutWarps);
     }
-    abort_flag = 0;
+    mbar_init(&mma_done, 1);
+    abort_flag = keep_tmem = 0;
     n_loaded = n_used = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -836,6 +837,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
           }
       }
       if (!ok) abort_flag = 1;
+      mma_commit(&mma_done, elected);  // also of the products of a stage left half issued
     }
   } else if (warp >= kDrainWarps) {
     // ---- outputs: parities combined, scaled, stored
@@ -931,16 +933,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_pass(const __grid_constant__
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) {
-    *b.failed = 1;
-    *b.expired = 1;
-    __threadfence_system();
-    // a wait ran out: let the loads in flight land before the CTA exits
-    for (int i = n_used; i < n_loaded; ++i) (void)mbar_wait(&full_bar[i % kStages], (unsigned)((i / kStages) & 1));
-    if (n_used > 0) (void)mbar_wait(&empty_bar[(n_used - 1) % kStages], (unsigned)(((n_used - 1) / kStages) & 1));
+  if (threadIdx.x == 0) {
+    // the loads and products in flight, and their arrivals, end before the CTA does;
+    // products that never finish keep their tensor memory
+    if (abort_flag)
+      for (int i = n_used; i < n_loaded; ++i) (void)mbar_wait(&full_bar[i % kStages], (unsigned)((i / kStages) & 1));
+    keep_tmem = mbar_wait(&mma_done, 0) ? 0 : 1;
+    if (abort_flag || keep_tmem) {
+      *b.failed = 1;
+      *b.expired = keep_tmem ? 2 : 1;
+      __threadfence_system();
+    }
   }
   __syncthreads();
-  if (warp == kMmaWarp)
+  if (warp == kMmaWarp && !keep_tmem)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 

@@ -42,6 +42,11 @@ for name, call in calls.items():
         out[name] = str(e)
     out[name + " left"] = int(host[0]) + sum(int(w[0]) for w in words)
     call()  # and runs again
+host[0] = 2
+try:
+    calls["transform"]()
+except hosnwt.HosError as e:
+    out["lost"] = str(e)
 print(json.dumps(out))
 """
 
@@ -51,3 +56,4 @@ def test_expired_wait_is_reported_once(host_lib):
     assert out["words"] == 1
     for name in ("transform", "runge4_adapt2", "step", "advance", "advance_many", "solveHOS2"):
         assert "(CUDA)" in out[name] and ("ran out" in out[name] or name == "advance_many") and out[name + " left"] == 0, (name, out)
+    assert "must not be used further" in out["lost"]
