@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "tank.h"
+#include "modes.h"
 
 namespace hos {
 
@@ -1025,18 +1026,16 @@ __global__ void k_phiadd_q(const double* __restrict__ a1, const double* __restri
 }
 
 // phiadd_SL (3-D): contraction over i3 at z = eta of the y-transformed B_q.
-// kx_add(i3) = (2 i3 + 1) pi / 4: cos / sin(kx_add(i3) (eta + 1)) by rotations
-// of 2 phi, phi = pi (eta + 1) / 4, from one sincos per kRestart modes, as in the
-// 1-D tank (a sincos per mode and point held the FP64 pipe for 546 us a call on
-// a 513 x 257 tank; its own error, the rounding of an angle of up to 100, is what
-// the rotations accumulate).  CY threads share the modes of a point where the
-// points alone are too few for the SMs.
+// cos / sin(kx_add(i3) (eta + 1)) by rotations, restarted every kRestart modes
+// (modes.h; a sincos per mode and point held the FP64 pipe for 546 us a call on
+// a 513 x 257 tank).  CY threads share the modes of a point where the points alone
+// are too few for the SMs.
 constexpr int kRestart = 32;
 template <int CY>
 __global__ void __launch_bounds__(128) k_phiadd_contract(
-    const double* __restrict__ eta, const double* __restrict__ kx_add, const double* __restrict__ Bt,
-    const double* __restrict__ Bx, const double* __restrict__ By, const double* __restrict__ Bz,
-    const double* __restrict__ Bp, int n1, int n2, int n3a, double* phix, double* phiy, double* phiz, double* phit,
+    const double* __restrict__ eta, double u, const double* __restrict__ Bt, const double* __restrict__ Bx,
+    const double* __restrict__ By, const double* __restrict__ Bz, const double* __restrict__ Bp, int n1, int n2,
+    int n3a, double* phix, double* phiy, double* phiz, double* phit,
     double* phi) {
   constexpr int CX = 128 / CY;
   __shared__ double r[CY > 1 ? 5 : 1][CY][CX];
@@ -1051,11 +1050,12 @@ __global__ void __launch_bounds__(128) k_phiadd_contract(
     const int ch = (n3a + CY - 1) / CY;
     const int a = ty * ch, b = min(n3a, a + ch);
     const long long base = i1 + (long long)n1 * n3a * i2;
+    auto sin_cos_pi = [](double x, double* s, double* c) { sincospi(x, s, c); };
     double s2, c2;
-    sincos(2.0 * kx_add[0] * e1, &s2, &c2);
+    mode_start(2.0 * u, e1, sin_cos_pi, s2, c2);
     for (int g = a; g < b; g += kRestart) {
       double s, c;
-      sincos(kx_add[g] * e1, &s, &c);
+      mode_start((2 * g + 1) * u, e1, sin_cos_pi, s, c);
       const int ge = min(b, g + kRestart);
 #pragma unroll 4
       for (int i3 = g; i3 < ge; ++i3) {
@@ -1065,9 +1065,7 @@ __global__ void __launch_bounds__(128) k_phiadd_contract(
         sy = fma(c, __ldg(By + o), sy);
         sz = fma(s, __ldg(Bz + o), sz);
         sp = fma(c, __ldg(Bp + o), sp);
-        const double cn = c * c2 - s * s2;
-        s = s * c2 + c * s2;
-        c = cn;
+        mode_next(s2, c2, s, c);
       }
     }
   }
@@ -1754,11 +1752,12 @@ void enqueue_rhs(Ctx& c, const double* y, double* k, bool rk_mode, cudaStream_t 
         for (int q = 0; q < 5; ++q) ys.push_back(YReq{d.Q[q], d.B[q], q == 2 ? 1 : 0});
         launch_y_f2s(W.tb, ys, lines, lines, lines, sw);
       }
-      // a point's modes shared by eight threads below 150 k points: 8192 points
-      // 66 us in one thread each with a sincos per mode
+      // a point's modes shared by eight threads below 32768 points, which one thread
+      // each would leave in fewer than two CTAs per SM: 8192 points took 66 us in one
+      // thread each with a sincos per mode
       auto contract = [&](auto kern, int cx) {
         launch_pdl(kern, dim3((unsigned)((nN + cx - 1) / cx)), dim3(128), 0, sw, (const double*)d.eta_sp,
-                   (const double*)d.kx_add, (const double*)d.B[0], (const double*)d.B[1], (const double*)d.B[2],
+                   0.5 / P.l_add, (const double*)d.B[0], (const double*)d.B[1], (const double*)d.B[2],
                    (const double*)d.B[3], (const double*)d.B[4], n1, n2, P.n3a, d.phix_add, d.phiy_add, d.phiz_add,
                    d.phit_add, d.phi_add);
       };
