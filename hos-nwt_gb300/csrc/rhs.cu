@@ -20,8 +20,9 @@
 #include <utility>
 #include <vector>
 
-#include "tank.h"
+#include "division.h"
 #include "modes.h"
+#include "tank.h"
 
 namespace hos {
 
@@ -173,16 +174,6 @@ struct PowArgs {
   double inv[16];  // 1 / (j + 1) rounded
   int j0, j1;
 };
-// v / d from r = 1 / d rounded: q = v r, corrected by its exact remainder
-// (Markstein, 1990): three operations in place of a division's dozen, which at
-// 64 issue cycles each held the steep tank's k_pow_run at 895 us a call.  A v
-// whose remainder could underflow, or that is not finite, is divided.
-__device__ __forceinline__ double div_by(double v, double d, double r) {
-  const int e = (__double2hiint(v) >> 20) & 0x7ff;
-  if (e < 64 || e == 0x7ff) return v / d;
-  const double q = v * r;
-  return fma(fma(-d, q, v), r, q);
-}
 __global__ void k_pow_run(PowArgs a, long long n) {
   pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;

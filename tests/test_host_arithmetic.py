@@ -1,5 +1,6 @@
 """Arithmetic that the kernels share with a host program built from the same
-headers: the vertical modes of the wavemaker potential by rotations (modes.h)."""
+headers: the vertical modes of the wavemaker potential by rotations (modes.h), the
+division by an order (division.h)."""
 import os
 import shutil
 import subprocess
@@ -72,3 +73,49 @@ def test_modes_by_rotations(tmp_path):
     direct cos(kx_add e) is; and no mode by more than 32 rotations can err (two
     rounded factors and three roundings of 2^-53 each, 5e-16: 1.6e-14)."""
     _run(tmp_path, MODES)
+
+
+DIVISION = r"""
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <initializer_list>
+#include "division.h"
+static double bits(unsigned long long b) {
+  double v;
+  std::memcpy(&v, &b, 8);
+  return v;
+}
+int main() {
+  unsigned long long bad = 0, n = 0, seed = 7;
+  auto look = [&](double v, double d) {
+    const double a = hos::div_by(v, d, 1.0 / d), b = v / d;
+    bad += std::memcmp(&a, &b, 8) != 0 && !(a != a && b != b);
+    ++n;
+  };
+  for (int d = 1; d <= 17; ++d) {
+    // exponents on both sides of the limit, the ends of the range, what is not finite
+    for (unsigned long long e : {0ULL, 1ULL, 2ULL, 53ULL, 62ULL, 63ULL, 64ULL, 65ULL, 1000ULL, 1022ULL, 1023ULL, 1500ULL, 2045ULL, 2046ULL, 2047ULL})
+      for (int k = 0; k < 4000; ++k) {
+        seed = seed * 6364136223846793005ULL + 1442695040888963407ULL;
+        const unsigned long long m = k == 0 ? 0 : (k == 1 ? 0xfffffffffffffULL : seed >> 12);
+        look(bits((e << 52) | m), d);
+        look(bits((1ULL << 63) | (e << 52) | m), d);
+      }
+    // quotients next to the middle of two doubles, and exact ones
+    for (int k = 0; k < 20000; ++k) {
+      seed = seed * 6364136223846793005ULL + 1442695040888963407ULL;
+      const double q = bits((1023ULL << 52) | (seed >> 12));
+      const double v = q * d, w = std::fma(q, (double)d, 0x1p-53 * d);
+      for (double x : {v, w, std::nextafter(v, 0.0), std::nextafter(v, 99.0), std::nextafter(w, 0.0), std::nextafter(w, 99.0)}) look(x, d);
+    }
+  }
+  std::printf("%llu of %llu differ\n", bad, n);
+  return bad != 0;
+}
+"""
+
+
+def test_division_by_an_order(tmp_path):
+    """The bits of v / d for d = 1 to 17."""
+    _run(tmp_path, DIVISION)
