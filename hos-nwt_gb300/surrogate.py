@@ -79,6 +79,8 @@ def gemm_bf16(A, B):
     Transposed views are read in place; K is zero-padded to a multiple of 8
     where an operand has it contiguous (the TMA row-stride rule)."""
     torch = _torch()
+    if A.shape[1] != B.shape[1]:  # a view read in place has the other's terms as its rows
+        raise hosnwt.HosError(f"gemm_bf16: operands of {A.shape[1]} and {B.shape[1]} terms")
     A = A if A.dtype == torch.bfloat16 else A.to(torch.bfloat16)
     B = B if B.dtype == torch.bfloat16 else B.to(torch.bfloat16)
     M, K = A.shape
