@@ -126,13 +126,13 @@ struct AxisJob {
   int ta, tb;                // term range [ta, tb) (interior terms or symmetric pairs)
   double* part;              // nlines * ntile * nchunk * 64 partial sums (nchunk > 1)
   unsigned int* cnt;         // nlines * ntile arrival counters (nchunk > 1)
-  // two-level passes (REDFT00 / RODFT00 kinds with D = A * B)
   // tensor-core passes: maxima over the lines that an x pass leaves for the y
   // pass that reads its output (high words of |.|), or null
   unsigned* cmax;
   const unsigned* lmax;
   const struct TcMat* tc;    // its matrix when the job runs on the tensor cores
   int tc_decided;            // 1: a y pass that goes as its x pass does
+  // two-level passes (REDFT00 / RODFT00 kinds with D = A * B)
   int A, B;                  // 0 when the direct sum is used
   double* cs;                // nlines * B * (A + 1) * 2 partial cos/sin sums
 };

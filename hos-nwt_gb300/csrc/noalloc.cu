@@ -11,8 +11,8 @@
 // The array holds the quarter-wave twiddle table and the partial sums and
 // arrival counters of the split transform sums.  It is shared by every call:
 // calls that overlap on the GPU (two streams, or two host threads) race on it
-// and give wrong results; serialise them.  Each call clears the counters and
-// rebuilds the table before its transform.
+// and give wrong results; serialise them.  Each call rebuilds the table before its
+// transform, and clears the counters where a sum may be split.
 #include <cuda_runtime.h>
 
 #include <mutex>

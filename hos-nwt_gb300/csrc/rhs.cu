@@ -1400,7 +1400,7 @@ struct Enq {
   template <typename K, typename... A>
   void ew(K kern, long long n, A... a) {
     if (n <= 0) return;
-    const int t = n <= 148LL * kEW ? kTrig : kEW;
+    const int t = n <= (long long)tb.nsm * kEW ? kTrig : kEW;
     launch_pdl(kern, dim3(nblk(n, t)), dim3(t), 0, st, a...);
   }
   template <typename K, typename... A>

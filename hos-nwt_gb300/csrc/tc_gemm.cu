@@ -43,7 +43,10 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 64;         // one 128-byte swizzle atom of BF16
 // stages of the ring: 4 let two CTAs share an SM; where every CTA has an SM of
-// its own the ring takes what fits
+// its own the ring takes what fits.  Over 128 to 6000 rows, 16 to 512 columns and 264
+// to 2056 terms that is within 1.2 % of four stages for short sums and few tiles, and
+// 4 to 20 % faster from 320 terms on 6000 rows and 768 on 2500 (6000 x 16 over 2056
+// terms 13.3 -> 11.1 us, 2500 x 64 over 1024 9.3 -> 8.1 us)
 constexpr int kStagesFew = 4;
 template <int BN>
 constexpr int kStagesDeep = BN > 64 ? 6 : 8;

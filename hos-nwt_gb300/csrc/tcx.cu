@@ -1213,7 +1213,8 @@ const TcMat* tc_matrix_of(const AxisJob& J, const Tables& tb) {
 // goes if its digits and products take less than its other passes, and all
 // of them together if they still do with the three launches of a pass.  The times
 // (us), measured on GB300: 6 ps per digit set (a y pass without maxima 12),
-// 17 us per pass for the launches and their latencies.  On both sides of the
+// 17 us per pass for the launches and their latencies, 8 us for those of a pass
+// elsewhere (pass_time counts its work alone).  On both sides of the
 // line (one field of the dealiased grid, both passes): 258 x 66 points 37
 // against 18 us by the FFT, 770 x 194 points 49 against 40, 642 x 627 points 59
 // against 77, 1282 x 642 points 93 against 128, 4100 x 2052 points 985 against 1920.

@@ -619,7 +619,7 @@ __device__ __forceinline__ double flip_if(double x, bool neg) {
 // input, truncated outputs) the slices run over u = x_j + x_{D-j} or v = x_j -
 // x_{D-j}.  D = 257, one line: 5.8 us by axis_pass_lanes_k (9 CTAs), 3.6 us here.
 constexpr int kDirThreads = 128;
-constexpr int kDirMaxD = 4200;      // table and inputs within 100 KB
+constexpr int kDirMaxD = 4200;      // table and inputs within 68 KB: three CTAs per SM
 constexpr int kDirMaxLines = 8;     // more lines fill the SMs by axis_pass_lanes_k
 __host__ __device__ inline int dir_terms(const AxisJob& J) {  // lane terms of the sum
   return J.mode == 2 ? J.D / 2 + 1 : (J.jhi < J.nin ? J.jhi : J.nin);
